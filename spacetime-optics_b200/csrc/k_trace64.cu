@@ -32,6 +32,7 @@
 #include <cuda_runtime.h>
 
 #include "so_emission.cuh"
+#include "so_fast64.cuh"
 #include "so_launch.h"
 
 namespace so {
@@ -44,7 +45,7 @@ struct Ray64 {
     RayC c;
     double y[6], k1[6];
     double h, trans, psi;
-    double pp0, pp1, pp2;
+    double sn;  // sin(theta) of y (radio)
     float acc[4];
     int ncross, nacc, natt, it, nflow;
 };
@@ -112,14 +113,7 @@ __device__ __forceinline__ void ray_init(Ray64& R, const so_scene& S, const so_f
     R.psi = 0.0;
     R.ncross = R.nacc = R.natt = R.it = R.nflow = 0;
     R.acc[0] = R.acc[1] = R.acc[2] = R.acc[3] = 0.f;
-    if (VAR == VAR_RADIO) {
-        double sp = sqrt(fmax(fma(-R.y[2], R.y[2], 1.0), 0.0));
-        double s4, c4;
-        sincos(R.y[4], &s4, &c4);
-        R.pp0 = sp * c4;
-        R.pp1 = sp * s4;
-        R.pp2 = R.y[2];
-    }
+    if (VAR == VAR_RADIO) R.sn = sin_of(R.y[2]);
 }
 
 enum Stage : int { ST_REJECTED = 0, ST_ACCEPTED = 1, ST_DONE = 2 };
@@ -158,14 +152,16 @@ __device__ __forceinline__ int ray_attempt(Ray64& R, const so_scene& S, bool emi
     ++R.it;
     double hc = R.h;
     if (VAR == VAR_RADIO && S.flow_on && R.y[0] < S.r_flow_max) {
-        double s = sqrt(fmax(fma(-R.y[2], R.y[2], 1.0), 0.0));
-        double cap = S.step_frac * fmin(R.y[0] / (fabs(R.y[1]) + 1e-30), fmax(s, 0.05) / (fabs(R.y[3]) + 1e-30));
-        hc = fmin(hc, cap);
+        // the smaller of r / |r'| and max(sin, 0.05) / |u'|, compared by products (dp54_fast)
+        const double q0 = fabs(R.y[1]) + 1e-30, q1 = fabs(R.y[3]) + 1e-30, s5 = R.sn > 0.05 ? R.sn : 0.05;
+        const bool rad = R.y[0] * q1 < s5 * q0;
+        const double cap = S.step_frac * fast_div(rad ? R.y[0] : s5, rad ? q0 : q1);
+        hc = cap < hc ? cap : hc;
     } else if (VAR != VAR_VACUUM && S.disk_on) {
-        hc = fmin(hc, 0.3 / (fabs(R.y[3]) + 1e-30));
+        hc = fmin(hc, fast_div(0.3, fabs(R.y[3]) + 1e-30));
     }
     ++R.natt;
-    double err = dp54(R.c, R.y, R.k1, hc, S.tol, yn, k7);
+    double err = dp54_attempt(R.c, R.y, R.k1, hc, S.tol, yn, k7);
     *hc_out = hc;
     *err_out = err;
     if (!(err <= 1.0)) {
@@ -174,19 +170,9 @@ __device__ __forceinline__ int ray_attempt(Ray64& R, const so_scene& S, bool emi
     }
     ++R.nacc;
     if (VAR == VAR_RADIO) {
-        double sn = sqrt(fmax(fma(-yn[2], yn[2], 1.0), 0.0));
-        double s4, c4;
-        sincos(yn[4], &s4, &c4);
-        double pn0 = sn * c4, pn1 = sn * s4, pn2 = yn[2];
-        double cx = fma(R.pp1, pn2, -(R.pp2 * pn1));
-        double cy = fma(R.pp2, pn0, -(R.pp0 * pn2));
-        double cz = fma(R.pp0, pn1, -(R.pp1 * pn0));
-        double cc = fma(cz, cz, fma(cy, cy, cx * cx));
-        double dd = fma(R.pp2, pn2, fma(R.pp1, pn1, R.pp0 * pn0));
-        R.psi += atan2(sqrt(cc), dd);
-        R.pp0 = pn0;
-        R.pp1 = pn1;
-        R.pp2 = pn2;
+        const double sn = sin_of(yn[2]);
+        R.psi += swept_angle(R.y[2], R.sn, yn[2], sn, yn[4] - R.y[4]);
+        R.sn = sn;
     }
     if ((R.y[2] > 0.0) != (yn[2] > 0.0)) {
         ++R.ncross;
@@ -261,8 +247,8 @@ __device__ __forceinline__ int ray_commit(Ray64& R, const so_scene& S, const so_
         R.y[i] = yn[i];
         R.k1[i] = k7[i];
     }
-    project_radial(R.c, R.y, R.k1);
-    R.h = accept_step(hc, err);
+    project_radial_fast(R.c, R.y, R.k1);
+    R.h = accept_step_fast(hc, err);
     if (R.y[0] < S.r_stop) {
         *fate = -1;
         return 1;

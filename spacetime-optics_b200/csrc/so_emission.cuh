@@ -9,7 +9,7 @@
 // rsqrtf of sheared_noise is written 1/sqrtf and __expf is expf so that the CPU oracle can follow the
 // same operations.
 #pragma once
-#include "so_kerr.cuh"
+#include "so_fast64.cuh"
 #include "so_launch.h"
 
 namespace so {
@@ -217,19 +217,24 @@ struct ModesSmem {
 // the raw coordinate time is ~ -rcam at the hole, which would put a factor rcam on every rounding
 // error of the advected phase.
 //
+// Whether a vertical profile exp(-zh^2 / 2) with zh^2 = u2 / w2 can reach 1e-7: flow_step's own test
+// without its exponential and quotient, a hair (1e-9) wider.  A step let through by the hair alone is
+// one that flow_step returns from: it emits nothing and transmits exactly 1.
+__device__ __forceinline__ bool profile_wants(double u2, double w2) { return !(u2 > 32.23619133 * w2); }
+
 // Where the torus turbulence is needed for a flow step at (r, u, phi, t): false when flow_step
 // returns before using it (only those flow steps can change the transfer); else the advected
 // azimuth phc of the sum's position.
 __device__ __forceinline__ bool torus_phase(const so_scene& S, const TorusParams& tp, double rcam, double r, double u,
                                             double phi, double t, double* phc) {
     if (!tp.on || tp.n_modes <= 0) return false;
-    double s2 = fmax(fma(-u, u, 1.0), 1e-12), s = sqrt(s2);
+    double s2 = fmax(fma(-u, u, 1.0), 1e-12), s = fast_sqrt(s2);
     double R = r * s;
     if (r > S.r_flow_max || R < 1e-3) return false;
-    double zh = u / tp.h_sph;
-    if (exp(-0.5 * zh * zh) < 1e-7) return false;
-    double Omf = S.flow_kep * keplerian_omega(S.a, fmax(R, S.r_isco));
-    *phc = phi - Omf * (t + (rcam - r + 2.0 * log(rcam / r)));
+    if (!profile_wants(u * u, tp.h_sph * tp.h_sph)) return false;
+    const double Rk = fmax(R, S.r_isco);
+    double Omf = S.flow_kep * fast_rcp(fma(Rk, fast_sqrt(Rk), S.a));
+    *phc = phi - Omf * (t + (rcam - r + 2.0 * log(fast_div(rcam, r))));
     return true;
 }
 // The Cartesian position (X, Y, Z) of the sum at (r, u) and advected azimuth phc.
@@ -291,24 +296,17 @@ __device__ __forceinline__ float baked_sample(const so_scene& S, const float* fi
 }
 
 // Whether flow_step on the reference flow model (no torus) can change the transfer at (r, u): its
-// first two returns, in its own arithmetic.  A step for which this is false emits nothing and
-// transmits exactly 1.
+// first two returns.  A step for which this is false emits nothing and transmits exactly 1.
 __device__ __forceinline__ bool flow_wants(const so_scene& S, double r, double u) {
-    double s2 = fmax(fma(-u, u, 1.0), 1e-12), s = sqrt(s2);
-    double R = r * s, z = r * u;
-    if (r > S.r_flow_max || R < 1e-3) return false;
-    double zh = z / (S.h_r * R);
-    return !(exp(-0.5 * zh * zh) < 1e-7);
+    const double s2 = fmax(fma(-u, u, 1.0), 1e-12);
+    // R^2 = r^2 sin^2, and zh = z / (h R) = u / (h sin)
+    return !(r > S.r_flow_max) && !(r * r * s2 < 0.999999999e-6) && profile_wants(u * u, S.h_r * S.h_r * s2);
 }
 
-// The same for the torus plasma (flow_step's torus branch: outside the flow region, or the vertical
-// profile exp(-(u / h_sph)^2 / 2) below 1e-7).
+// The same for the torus plasma (flow_step's torus branch: zh = u / h_sph).
 __device__ __forceinline__ bool torus_wants(const so_scene& S, const TorusParams& tp, double r, double u) {
-    double s2 = fmax(fma(-u, u, 1.0), 1e-12), s = sqrt(s2);
-    double R = r * s;
-    if (r > S.r_flow_max || R < 1e-3) return false;
-    double zh = u / tp.h_sph;
-    return !(exp(-0.5 * zh * zh) < 1e-7);
+    const double s2 = fmax(fma(-u, u, 1.0), 1e-12);
+    return !(r > S.r_flow_max) && !(r * r * s2 < 0.999999999e-6) && profile_wants(u * u, tp.h_sph * tp.h_sph);
 }
 
 // flow_step with the torus turbulence sum `delta` at this point already evaluated (torus_position).
