@@ -34,6 +34,7 @@
 #include "so_emission.cuh"
 #include "so_fast64.cuh"
 #include "so_launch.h"
+#include "so_packed32.cuh"
 
 namespace so {
 
@@ -775,48 +776,47 @@ cudaError_t launch_turb64_records(const TraceLaunch& L, int num_sms, cudaStream_
 }
 
 // The mixed form of the deferred sums (FP64 geometry, FP32 turbulence sums, as the tracer's EMIT32):
-// FP32 SFU cosines at every record of a recording pass, the modes folded to FP32 in constant memory
-// (the kernel parameter), kTurb32RecP positions per thread at slots c0 + t + 256 q of a block's
-// chunk, each position formed in FP64 from (r, u, azimuth) as the tracer forms it and rounded to
-// FP32.  The sum (in mode order) goes to the record's slot [2] as the FP64 sums do.  Twelve
-// positions per mode load (80 registers): the photon-ring batch at 2.15 Mrays/s against 2.09 with
-// eight (74 registers).
-constexpr int kTurb32RecP = 12;
-__global__ void __launch_bounds__(256) k_turb32_rec64(const TraceLaunch L, const __grid_constant__ TurbModes M) {
+// FP32 cosines at every record of a recording pass, the modes folded to FP32 in constant memory (the
+// kernel parameter), kTurb32RecP positions per thread in pairs (mode_sums2) at slots c0 + t + 256 q of a
+// block's chunk, each position formed in FP64 from (r, u, azimuth) as the tracer forms it and rounded
+// to FP32.  The sum (in mode order) goes to the record's slot [2] as the FP64 sums do.
+constexpr int kTurb32RecP = 8;
+__global__ void __launch_bounds__(256, 4) k_turb32_rec64(const TraceLaunch L, const __grid_constant__ TurbModes M) {
     unsigned long long used = *(volatile unsigned long long*)&L.rec64_ctl[0];
     if (used > (unsigned long long)L.seg_cap64) used = (unsigned long long)L.seg_cap64;
     const long long nslots = (long long)used * REC_SEG;
-    const int nm = M.n;
     constexpr int P = kTurb32RecP;
     const long long chunk = 256LL * P;
     for (long long c0 = (long long)blockIdx.x * chunk; c0 < nslots; c0 += (long long)gridDim.x * chunk) {
-        float x[P], y[P], z[P], acc[P];
-        bool live[P];
+        F2 x[P / 2], y[P / 2], z[P / 2], acc[P / 2];
+        unsigned live = 0;
 #pragma unroll
-        for (int q = 0; q < P; ++q) {
-            const long long slot = c0 + threadIdx.x + 256LL * q;
-            live[q] = slot < nslots && (int)(slot % REC_SEG) < (int)L.seg_meta64[slot / REC_SEG].y;
-            double X = 0.0, Y = 0.0, Z = 0.0;
-            if (live[q]) {
-                const double* rec = L.rec64 + (long long)L.rec64_w * slot;
-                torus_xyz(rec[0], rec[1], rec[2], &X, &Y, &Z);
+        for (int q = 0; q < P / 2; ++q) {
+            double X[2] = {0.0, 0.0}, Y[2] = {0.0, 0.0}, Z[2] = {0.0, 0.0};
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const long long slot = c0 + threadIdx.x + 256LL * (2 * q + e);
+                if (slot < nslots && (int)(slot % REC_SEG) < (int)L.seg_meta64[slot / REC_SEG].y) {
+                    const double* rec = L.rec64 + (long long)L.rec64_w * slot;
+                    torus_xyz(rec[0], rec[1], rec[2], &X[e], &Y[e], &Z[e]);
+                    live |= 1u << (2 * q + e);
+                }
             }
-            x[q] = (float)X;
-            y[q] = (float)Y;
-            z[q] = (float)Z;
-            acc[q] = 0.f;
+            x[q] = pack2((float)X[0], (float)X[1]);
+            y[q] = pack2((float)Y[0], (float)Y[1]);
+            z[q] = pack2((float)Z[0], (float)Z[1]);
+            acc[q] = both(0.f);
         }
-#pragma unroll 2
-        for (int m = 0; m < nm; ++m) {
-            const float4 k = M.k[m];
-            const float am = M.a[m];
+        mode_sums2<P / 2>(M, x, y, z, acc);
 #pragma unroll
-            for (int q = 0; q < P; ++q)
-                acc[q] = fmaf(am, __cosf(fmaf(k.z, z[q], fmaf(k.y, y[q], fmaf(k.x, x[q], k.w)))), acc[q]);
+        for (int q = 0; q < P / 2; ++q) {
+            float v[2];
+            unpack2(acc[q], &v[0], &v[1]);
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+                if ((live >> (2 * q + e)) & 1u)
+                    L.rec64[(long long)L.rec64_w * (c0 + threadIdx.x + 256LL * (2 * q + e)) + 2] = (double)v[e];
         }
-#pragma unroll
-        for (int q = 0; q < P; ++q)
-            if (live[q]) L.rec64[(long long)L.rec64_w * (c0 + threadIdx.x + 256LL * q) + 2] = (double)acc[q];
     }
 }
 

@@ -29,6 +29,7 @@
 
 #include "so_emission.cuh"
 #include "so_launch.h"
+#include "so_packed32.cuh"
 
 namespace so {
 
@@ -842,56 +843,56 @@ __device__ __forceinline__ Torus32 torus32_of(const TraceLaunch& L) {
 
 // Turbulence sum at every record slot in use: the records' positions (the tracer's in-line form:
 // R = r sqrt(max((1-u)(1+u), 1e-12)), x = R cos phi_c, y = R sin phi_c, z = r u), TURB_P positions
-// per thread, the modes read from constant memory (the kernel parameter M, the same address for the
-// whole warp: no shared-memory loads in the MIO queue that feeds the SFU), so every lane does the
-// same work and the SFU cosine is the bound (three FMAs, the cosine's scaling multiply, the cosine
-// and one FMA per mode and position).  Each mode's constant loads serve TURB_P positions: measured
-// on the 2048^2 frame, 8 positions (64 registers, 4 CTAs / SM) 142.6 ms at 0.85 of the SFU rate, 12
-// (80 registers, 3 CTAs) 134.0 ms at 0.90, 16 (126 registers, 2 CTAs) 142.3 ms.  Blocks take chunks
-// of TURB_P x 256 slots from a work counter, so SMs that also host the FP64 re-trace (on the other
-// stream) do less of it instead of finishing last.  Slots of a segment past its ray's last record
-// hold stale data; their sums are never read.
-constexpr int TURB_P = 12;
+// per thread in pairs (mode_sums2, so_packed32.cuh), the modes read from constant memory (the kernel
+// parameter M, the same address for the whole warp: no shared-memory loads in the MIO queue that
+// feeds the SFU), so every lane does the same work.  Blocks take chunks of TURB_P x 256 slots from a
+// work counter, so SMs that also host the FP64 re-trace (on the other stream) do less of it instead
+// of finishing last.  Slots of a segment past its ray's last record hold stale data; their sums are
+// never read.
+constexpr int TURB_P = 8;
 constexpr int TURB_CHUNK = TURB_P * 256;
-__global__ void __launch_bounds__(256) k_turb_records(const TraceLaunch L, const __grid_constant__ TurbModes M) {
-    const int nm = M.n;
+__global__ void __launch_bounds__(256, 4) k_turb_records(const TraceLaunch L, const __grid_constant__ TurbModes M) {
     __shared__ long long chunk;
     unsigned long long used = L.nlists[5];
     if (used > (unsigned long long)L.seg_cap) used = (unsigned long long)L.seg_cap;
     const long long nslots = (long long)used * REC_SEG;
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&L.nlists[10], used);
     for (;;) {
-        __syncthreads();  // modes loaded; the previous chunk index read by every thread
+        __syncthreads();  // the previous chunk index read by every thread
         if (threadIdx.x == 0) chunk = (long long)atomicAdd(&L.nlists[7], 1ull) * TURB_CHUNK;
         __syncthreads();
         const long long c0 = chunk;
         if (c0 >= nslots) break;
         const long long i = c0 + threadIdx.x;  // slots i + 256 q, q < TURB_P
-        float x[TURB_P], y[TURB_P], z[TURB_P], acc[TURB_P];
+        F2 x[TURB_P / 2], y[TURB_P / 2], z[TURB_P / 2], acc[TURB_P / 2];
 #pragma unroll
-        for (int q = 0; q < TURB_P; ++q) {
-            const long long j = min(i + q * 256, nslots - 1);
-            const float4 v = L.rec[j];
-            const float r = fabsf(v.x), u = v.y;
-            const float s2 = fmaxf((1.f - u) * (1.f + u), 1e-12f), Rc = r * sqrtf(s2);
-            float sp, cp;
-            __sincosf(v.z, &sp, &cp);
-            x[q] = Rc * cp;
-            y[q] = Rc * sp;
-            z[q] = r * u;
-            acc[q] = 0.f;
+        for (int q = 0; q < TURB_P / 2; ++q) {
+            float px[2], py[2], pz[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const long long j = min(i + (2 * q + e) * 256, nslots - 1);
+                const float4 v = L.rec[j];
+                const float r = fabsf(v.x), u = v.y;
+                const float s2 = fmaxf((1.f - u) * (1.f + u), 1e-12f), Rc = r * sqrtf(s2);
+                float sp, cp;
+                __sincosf(v.z, &sp, &cp);
+                px[e] = Rc * cp;
+                py[e] = Rc * sp;
+                pz[e] = r * u;
+            }
+            x[q] = pack2(px[0], px[1]);
+            y[q] = pack2(py[0], py[1]);
+            z[q] = pack2(pz[0], pz[1]);
+            acc[q] = both(0.f);
         }
-#pragma unroll 2
-        for (int m = 0; m < nm; ++m) {
-            const float4 k = M.k[m];
-            const float am = M.a[m];
+        mode_sums2<TURB_P / 2>(M, x, y, z, acc);
 #pragma unroll
-            for (int q = 0; q < TURB_P; ++q)
-                acc[q] = fmaf(am, __cosf(fmaf(k.z, z[q], fmaf(k.y, y[q], fmaf(k.x, x[q], k.w)))), acc[q]);
+        for (int q = 0; q < TURB_P / 2; ++q) {
+            float a, b;
+            unpack2(acc[q], &a, &b);
+            if (i + 2 * q * 256 < nslots) L.rec_delta[i + 2 * q * 256] = a;
+            if (i + (2 * q + 1) * 256 < nslots) L.rec_delta[i + (2 * q + 1) * 256] = b;
         }
-#pragma unroll
-        for (int q = 0; q < TURB_P; ++q)
-            if (i + q * 256 < nslots) L.rec_delta[i + q * 256] = acc[q];
     }
 }
 
@@ -1042,7 +1043,9 @@ void turb_modes_fold(const so_mode* modes, int n, TurbModes* out) {
     for (int i = 0; i < n; ++i) {
         const so_mode& m = modes[i];
         const double ph = m.phase - 2.0 * PI * floor(m.phase / (2.0 * PI) + 0.5);
-        out->k[i] = make_float4((float)m.kx, (float)m.ky, (float)m.kz, (float)ph);
+        const bool poly = i % TURB_POLY == TURB_POLY - 1;
+        const double f = poly ? 0.5 / PI : 1.0;
+        out->k[i] = make_float4((float)(m.kx * f), (float)(m.ky * f), (float)(m.kz * f), (float)(ph * f));
         out->a[i] = (float)m.amp;
     }
 }

@@ -222,7 +222,10 @@ cudaError_t launch_corner_uv(const so_scene* d_scene, long long n, const int8_t*
 cudaError_t launch_mip_half2(cudaSurfaceObject_t src, int sw, int sh, cudaSurfaceObject_t dst, int dw, int dh,
                              cudaStream_t st);
 // Fourier modes of the torus turbulence in FP32 (phase folded into (-pi, pi]), passed to the batched
-// sums as a kernel parameter (constant memory; up to SO_MAX_MODES = 1024, 20 KB).
+// sums as a kernel parameter (constant memory; up to SO_MAX_MODES = 1024, 20 KB).  The last of every
+// complete group of TURB_POLY modes has its wave vector and phase in turns (its cosine is taken on
+// the FMA pipe, so_packed32.cuh).
+constexpr int TURB_POLY = 8;
 struct TurbModes {
     float4 k[SO_MAX_MODES];  // kx, ky, kz, phase
     float a[SO_MAX_MODES];   // amplitude
