@@ -985,43 +985,6 @@ cudaError_t launch_transfer64(const TraceLaunch& L, int num_sms, cudaStream_t st
     return cudaGetLastError();
 }
 
-// Host launcher: grid = SMs x resident CTAs per SM (persistent; capped by L.ctas_per_sm), dynamic
-// shared memory for the mode table.  Returns the CUDA error of the launch.
-// Bake of the flow turbulence for the frame in d_frame (k_bake_turb, render.cu:449-460): slice k
-// holds exp(a n - a^2 / 2) of the sheared noise n at the retarded time t_ref(r) + delta_k, on cell
-// centres phi = 2 pi (i + 1/2) / 512, ln R uniform over [lr0, lr1] (192 cells), z / R uniform over
-// [-zmax, zmax] (48 cells).  One thread per cell, phi fastest (coalesced stores).
-__device__ __forceinline__ float bake_texel(const so_scene& S, const so_frame& F, const TurbBake& b, int i, int j,
-                                             int l, int k) {
-    const double phi = (i + 0.5) / TURB_NPHI * 2.0 * PI;
-    const double R = exp(S.turb_lr0 + (j + 0.5) / TURB_NLR * (S.turb_lr1 - S.turb_lr0));
-    const double z = (-1.0 + 2.0 * (l + 0.5) / TURB_NZ) * S.turb_zmax * R;
-    const double r = sqrt(fma(R, R, z * z));
-    const double t = (F.t - (F.r - r + 2.0 * log(F.r / r))) + b.delta[k];
-    const float n = sheared_noise(S, R, phi, z, t, S.flow_turb_scale, S.flow_tcorr, S.seed ^ 0x51f15eedu);
-    const float a = S.flow_turb_amp;
-    return __expf(a * n - 0.5f * a * a);
-}
-
-__global__ void __launch_bounds__(256) k_bake_turb(const so_scene* __restrict__ Sp, const so_frame* __restrict__ Fp,
-                                                   const TurbBake b, float* __restrict__ field) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int l = blockIdx.z % TURB_NZ, k = blockIdx.z / TURB_NZ;
-    if (i >= TURB_NPHI || j >= TURB_NLR) return;
-    field[(((size_t)k * TURB_NZ + l) * TURB_NLR + j) * TURB_NPHI + i] = bake_texel(*Sp, *Fp, b, i, j, l, k);
-}
-
-// The same texels into slice k's 3-D array through its surface (x = phi, y = ln R, z = z / R), for
-// the texture-unit fetch (render.cu:449-460 writes its slices the same way).
-__global__ void __launch_bounds__(256) k_bake_turb_surf(const so_scene* __restrict__ Sp,
-                                                        const so_frame* __restrict__ Fp, const TurbBake b,
-                                                        const SurfaceSet surf) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int l = blockIdx.z % TURB_NZ, k = blockIdx.z / TURB_NZ;
-    if (i >= TURB_NPHI || j >= TURB_NLR) return;
-    surf3Dwrite(bake_texel(*Sp, *Fp, b, i, j, l, k), surf.s[k], i * (int)sizeof(float), j, l);
-}
-
 // Pixel corners (k_corners, render.cu:40-52): corner (x, y) of a W x H frame at tangent-plane point
 // ((x - W/2) pix, (H/2 - y) pix), x in [0, W], y in [0, H].
 __global__ void k_corner_points(const so_frame* __restrict__ Fp, int W, int H, double* __restrict__ xs,
@@ -1075,20 +1038,8 @@ cudaError_t launch_mip_half2(cudaSurfaceObject_t src, int sw, int sh, cudaSurfac
     return cudaGetLastError();
 }
 
-cudaError_t launch_bake_turb(const so_scene* d_scene, const so_frame* d_frame, const TurbBake& b, float* field,
-                             cudaStream_t st) {
-    const dim3 block(32, 8), grid(TURB_NPHI / 32, TURB_NLR / 8, TURB_NZ * TURB_NT);
-    k_bake_turb<<<grid, block, 0, st>>>(d_scene, d_frame, b, field);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_bake_turb_surf(const so_scene* d_scene, const so_frame* d_frame, const TurbBake& b,
-                                  const SurfaceSet& surf, cudaStream_t st) {
-    const dim3 block(32, 8), grid(TURB_NPHI / 32, TURB_NLR / 8, TURB_NZ * TURB_NT);
-    k_bake_turb_surf<<<grid, block, 0, st>>>(d_scene, d_frame, b, surf);
-    return cudaGetLastError();
-}
-
+// Host launcher: grid = SMs x resident CTAs per SM (persistent; capped by L.ctas_per_sm), dynamic
+// shared memory for the mode table.  Returns the CUDA error of the launch.
 cudaError_t launch_trace64(const TraceLaunch& L, int variant, int num_sms, cudaStream_t st) {
     const int tpb = 128;
     const bool torus = variant == VAR_RADIO && L.torus && L.n_modes > 0;

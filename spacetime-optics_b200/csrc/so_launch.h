@@ -207,13 +207,13 @@ cudaError_t launch_route(const TraceLaunch& L, int all64, cudaStream_t st);
 cudaError_t launch_approach64(const TraceLaunch& L, long long n, int num_sms, cudaStream_t st);
 cudaError_t launch_trace32(const TraceLaunch& L, long long n, int variant, int num_sms, cudaStream_t st);
 cudaError_t launch_bake_turb(const so_scene* d_scene, const so_frame* d_frame, const TurbBake& b, float* field,
-                             cudaStream_t st);
+                             int num_sms, cudaStream_t st);
 // The same bake into TURB_NT 3-D float arrays through their surface objects (texture-fetch mode).
 struct SurfaceSet {
     cudaSurfaceObject_t s[TURB_NT];
 };
 cudaError_t launch_bake_turb_surf(const so_scene* d_scene, const so_frame* d_frame, const TurbBake& b,
-                                  const SurfaceSet& surf, cudaStream_t st);
+                                  const SurfaceSet& surf, int num_sms, cudaStream_t st);
 // Sky: tangent-plane points of the (W + 1) x (H + 1) pixel corners of the frame in d_frame, the
 // corners' escape (u, v) from the tracer's outputs, and one box-filtered half2 mip level.
 cudaError_t launch_corner_points(const so_frame* d_frame, int W, int H, double* x, double* y, cudaStream_t st);

@@ -364,12 +364,12 @@ int bake_turbulence(so_renderer* r, TraceLaunch& L) {
     if (r->turb_arr[0]) {
         SurfaceSet ss;
         for (int k = 0; k < TURB_NT; ++k) ss.s[k] = r->turb_surf[k];
-        SO_CK(r, launch_bake_turb_surf(r->d_scene, r->d_frame, r->tb, ss, r->st));
+        SO_CK(r, launch_bake_turb_surf(r->d_scene, r->d_frame, r->tb, ss, r->num_sms, r->st));
         L.turb_field = nullptr;
         return SO_OK;
     }
     if (!r->d_turb) return SO_OK;
-    SO_CK(r, launch_bake_turb(r->d_scene, r->d_frame, r->tb, r->d_turb, r->st));
+    SO_CK(r, launch_bake_turb(r->d_scene, r->d_frame, r->tb, r->d_turb, r->num_sms, r->st));
     L.turb_field = r->d_turb;
     return SO_OK;
 }
