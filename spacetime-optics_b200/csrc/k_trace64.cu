@@ -717,61 +717,129 @@ __global__ void __launch_bounds__(128, DEFER >= 1 ? 4 : 3) k_trace64(const Trace
     }
 }
 
-// Deferred FP64 turbulence: the sum at every record written by a recording pass of k_trace64, by the
-// same warp_sums arithmetic as the tracer's own sums (so the emission reads exactly the value the
-// tracer would have computed).  Each warp takes kTurb64PerPass consecutive slots at a time, the grid
-// strides over all slots of the segments taken; lane j turns slot j's (r, u, azimuth) into its
-// position and the warp shares it, and the slots past a chain's last record (the segment's count)
-// are summed at the origin and left unwritten.  The whole SM runs this kernel, without the tracer's
-// register load, so many more warps hide the FP64 latency of the cosine chains.
-// Records per warp pass: their cosines interleave.  Measured on the 1024^2 synchrotron frame: 2 per
-// pass (42 registers) 212 ms, 4 (62) 201 ms, 8 (118 registers, two 256-thread CTAs per SM) 167 ms.
-constexpr int kTurb64PerPass = 8;
-__global__ void __launch_bounds__(256) k_turb64_records(const TraceLaunch L) {
-    extern __shared__ double smem64[];
+// Deferred FP64 turbulence: the sum at every record written by a recording pass of k_trace64, equal bit
+// for bit to warp_sums (so the emission reads exactly the value the tracer would have computed).
+//
+// The FP64 pipe bounds it (16 FP64 instructions per mode and position).  warp_sums gives every lane its own
+// modes, so an FMA of the phase reads three different registers and the pipe starves on the
+// register file: 0.77 T mode-positions/s whatever the number of positions and warps.  Here a thread
+// owns kTurb64P positions and all threads read the same mode, a broadcast of 16-byte shared loads
+// whose values the positions reuse.  The 1024^2 synchrotron frame's sums: 181.8 -> 155.0 ms (0.95 T
+// mode-positions/s, 2.5 cycles per FP64 instruction against 2.2 of independent FMAs); with 4
+// positions 176 (unrolled twice 165), with 6 166, with 10 in CTAs of 128 172.
+//
+// The order of warp_sums is kept: partial sum l takes modes l, l + 32, l + 64, ..., and the butterfly
+// (xor 16, 8, 4, 2, 1) adds the partials as a balanced tree whose leaves are l in bit-reversed order.
+// Visiting l in that order, a binary counter of five pending subtrees per position adds the same
+// pairs.  Slots past a chain's last record (the segment's count) are summed at the origin and left
+// unwritten.
+constexpr int kTurb64P = 8;
+// acc[j] += w cos_turns(k . X_j + p), written stage by stage over the positions (the operations of
+// cos_turns, so_kerr.cuh), so that the P chains interleave.
+template <int P>
+__device__ __forceinline__ void add_mode(double kx, double ky, double kz, double p0, double w, const double* px,
+                                         const double* py, const double* pz, double* acc) {
+    const double magic = 6755399441055744.0;
+    double s[P], z[P], c[P];
+#define EACH for (int j = 0; j < P; ++j)
+#pragma unroll
+    EACH z[j] = fma(kx, px[j], p0);
+#pragma unroll
+    EACH z[j] = fma(ky, py[j], z[j]);
+#pragma unroll
+    EACH z[j] = fma(kz, pz[j], z[j]);
+#pragma unroll
+    EACH s[j] = fma(z[j], 2.0, magic);
+#pragma unroll
+    EACH z[j] = fma(s[j] - magic, -0.5, z[j]);
+#pragma unroll
+    EACH z[j] = z[j] * z[j];
+#pragma unroll
+    EACH c[j] = fma(0x1.1678f9078a9b3p-2, z[j], -0x1.b6957b54dd389p+0);
+    const double C[7] = {0x1.f9d254582ac30p+2,  -0x1.a6d1efc8c38bep+4, 0x1.e1f506813a321p+5, -0x1.55d3c7e3bfbf5p+6,
+                         0x1.03c1f081b5992p+6, -0x1.3bd3cc9be45dbp+4, 1.0};
+#pragma unroll
+    for (int i = 0; i < 7; ++i) {
+#pragma unroll
+        EACH c[j] = fma(c[j], z[j], C[i]);
+    }
+#pragma unroll
+    EACH acc[j] = fma(w, bitsd(dbits(c[j]) ^ ((dbits(s[j]) & 1ull) << 63)), acc[j]);
+#undef EACH
+}
+constexpr int kTurb64Threads = 256;
+constexpr int kModeStride = 6;  // doubles per mode in shared memory: k, phase, amplitude, pad
+__global__ void __launch_bounds__(kTurb64Threads) k_turb64_records(const TraceLaunch L) {
+    extern __shared__ __align__(16) double smem64[];
     const int n = L.n_modes;
-    const ModesSmem md = stage_modes64(smem64, L.modes, n);
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const so_mode m = L.modes[i];
+        double* q = smem64 + kModeStride * i;
+        q[0] = m.kx * kInvTwoPi;
+        q[1] = m.ky * kInvTwoPi;
+        q[2] = m.kz * kInvTwoPi;
+        q[3] = m.phase * kInvTwoPi;
+        q[4] = m.amp;
+    }
     __syncthreads();
     unsigned long long used = *(volatile unsigned long long*)&L.rec64_ctl[0];
     if (used > (unsigned long long)L.seg_cap64) used = (unsigned long long)L.seg_cap64;
     const long long nslots = (long long)used * REC_SEG;
-    const int lane = threadIdx.x & 31;
-    const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-    constexpr int P = kTurb64PerPass;
-    for (long long s0 = P * warp; s0 < nslots; s0 += P * nwarps) {
-        const long long mine_slot = s0 + lane;
-        const bool live = lane < P && mine_slot < nslots &&
-                          (int)(mine_slot % REC_SEG) < (int)L.seg_meta64[mine_slot / REC_SEG].y;
-        double X = 0.0, Y = 0.0, Z = 0.0;
-        double* rec = L.rec64 + (long long)L.rec64_w * (live ? mine_slot : 0);
-        if (live) torus_xyz(rec[0], rec[1], rec[2], &X, &Y, &Z);
-        double px[P], py[P], pz[P], acc[P];
+    constexpr int P = kTurb64P;
+    constexpr long long chunk = (long long)P * kTurb64Threads;
+    for (long long c0 = (long long)blockIdx.x * chunk; c0 < nslots; c0 += (long long)gridDim.x * chunk) {
+        double px[P], py[P], pz[P], acc[P], sub[5][P];
+        unsigned live = 0;
 #pragma unroll
         for (int j = 0; j < P; ++j) {
-            px[j] = __shfl_sync(FULL, X, j);
-            py[j] = __shfl_sync(FULL, Y, j);
-            pz[j] = __shfl_sync(FULL, Z, j);
+            const long long slot = c0 + threadIdx.x + (long long)kTurb64Threads * j;
+            px[j] = py[j] = pz[j] = 0.0;
+            if (slot < nslots && (int)(slot % REC_SEG) < (int)L.seg_meta64[slot / REC_SEG].y) {
+                const double* rec = L.rec64 + (long long)L.rec64_w * slot;
+                torus_xyz(rec[0], rec[1], rec[2], &px[j], &py[j], &pz[j]);
+                live |= 1u << j;
+            }
         }
-        warp_sums<P>(md, n, px, py, pz, acc);
-        double mine = acc[0];
+#pragma unroll 1
+        for (unsigned b = 0; b < 32; ++b) {
 #pragma unroll
-        for (int j = 1; j < P; ++j)
-            if (lane == j) mine = acc[j];
-        if (live) rec[2] = mine;
+            for (int j = 0; j < P; ++j) acc[j] = 0.0;
+#pragma unroll 1
+            for (int i = (int)(__brev(b) >> 27); i < n; i += 32) {
+                const double2* q = reinterpret_cast<const double2*>(smem64 + kModeStride * i);
+                const double2 k01 = q[0], k23 = q[1];
+                const double w = smem64[kModeStride * i + 4];
+                add_mode<P>(k01.x, k01.y, k23.x, k23.y, w, px, py, pz, acc);
+            }
+#pragma unroll
+            for (int lev = 0; lev < 5; ++lev) {
+                if (!((b >> lev) & 1u)) {
+#pragma unroll
+                    for (int j = 0; j < P; ++j) sub[lev][j] = acc[j];
+                    break;
+                }
+#pragma unroll
+                for (int j = 0; j < P; ++j) acc[j] = sub[lev][j] + acc[j];
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < P; ++j) {
+            const long long slot = c0 + threadIdx.x + (long long)kTurb64Threads * j;
+            if ((live >> j) & 1u) L.rec64[(long long)L.rec64_w * slot + 2] = acc[j];
+        }
     }
 }
 
 cudaError_t launch_turb64_records(const TraceLaunch& L, int num_sms, cudaStream_t st) {
-    const size_t smem = (size_t)L.n_modes * 5 * sizeof(double);
+    const size_t smem = (size_t)L.n_modes * kModeStride * sizeof(double);
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(k_turb64_records, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
     int per_sm = 1;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_turb64_records, 256, smem);
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_turb64_records, kTurb64Threads, smem);
     if (e != cudaSuccess) return e;
-    k_turb64_records<<<num_sms * (per_sm > 0 ? per_sm : 1), 256, smem, st>>>(L);
+    k_turb64_records<<<num_sms * (per_sm > 0 ? per_sm : 1), kTurb64Threads, smem, st>>>(L);
     return cudaGetLastError();
 }
 
