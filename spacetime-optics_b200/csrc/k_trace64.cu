@@ -104,6 +104,13 @@ __device__ __forceinline__ JobPlace job_place(const TraceLaunch& L, long long jo
     return q;
 }
 
+// Where the steps read their scene values: the launch descriptor (HOT) or the ray's scene.
+template <bool HOT>
+__device__ __forceinline__ auto& step_scene(const TraceLaunch& L, const so_scene* S) {
+    if constexpr (HOT) return L.hot;
+    else return *S;
+}
+
 template <int VAR>
 __device__ __forceinline__ void ray_init(Ray64& R, const so_scene& S, const so_frame& F, double x, double yv) {
     so_vec3 d = view_dir(F, x, yv);
@@ -142,27 +149,27 @@ __device__ __forceinline__ void list_out(const so_rays_out& o, long long job, in
 // controller on rejection, swept angle, equatorial crossing (with the disk).  On acceptance the new
 // state is in yn / k7 and the ray continues in ray_commit.  Without `emit` (the recording pass of the
 // deferred turbulence) the disk is not shaded, so no ray ends on its opacity.
-template <int VAR>
-__device__ __forceinline__ int ray_attempt(Ray64& R, const so_scene& S, bool emit, double* yn, double* k7,
+template <int VAR, bool TIME, class Scene>
+__device__ __forceinline__ int ray_attempt(Ray64& R, const Scene& H, const so_scene& S, bool emit, double* yn, double* k7,
                                            double* hc_out, double* err_out, int* fate, double* cross_r,
                                            double* cross_g) {
-    if (R.it >= S.max_steps) {
+    if (R.it >= H.max_steps) {
         *fate = 0;
         return ST_DONE;
     }
     ++R.it;
     double hc = R.h;
-    if (VAR == VAR_RADIO && S.flow_on && R.y[0] < S.r_flow_max) {
+    if (VAR == VAR_RADIO && H.flow_on && R.y[0] < H.r_flow_max) {
         // the smaller of r / |r'| and max(sin, 0.05) / |u'|, compared by products (dp54_fast)
         const double q0 = fabs(R.y[1]) + 1e-30, q1 = fabs(R.y[3]) + 1e-30, s5 = R.sn > 0.05 ? R.sn : 0.05;
         const bool rad = R.y[0] * q1 < s5 * q0;
-        const double cap = S.step_frac * fast_div(rad ? R.y[0] : s5, rad ? q0 : q1);
+        const double cap = H.step_frac * fast_div(rad ? R.y[0] : s5, rad ? q0 : q1);
         hc = cap < hc ? cap : hc;
-    } else if (VAR != VAR_VACUUM && S.disk_on) {
+    } else if (VAR != VAR_VACUUM && H.disk_on) {
         hc = fmin(hc, fast_div(0.3, fabs(R.y[3]) + 1e-30));
     }
     ++R.natt;
-    double err = dp54_attempt(R.c, R.y, R.k1, hc, S.tol, yn, k7);
+    double err = dp54_attempt<TIME>(R.c, R.y, R.k1, hc, H.tol, yn, k7);
     *hc_out = hc;
     *err_out = err;
     if (!(err <= 1.0)) {
@@ -178,7 +185,7 @@ __device__ __forceinline__ int ray_attempt(Ray64& R, const so_scene& S, bool emi
     if ((R.y[2] > 0.0) != (yn[2] > 0.0)) {
         ++R.ncross;
         const bool rec = cross_r != nullptr && R.ncross <= 3;
-        const bool disk = VAR != VAR_VACUUM && S.disk_on && emit;
+        const bool disk = VAR != VAR_VACUUM && H.disk_on && emit;
         if (disk || rec) {
             double lo = 0.0, hi = 1.0, u0 = R.y[2], u1 = yn[2], m0 = R.y[3] * hc, m1 = yn[3] * hc;
             for (int b = 0; b < 40; ++b) {
@@ -220,12 +227,13 @@ __device__ __forceinline__ int ray_attempt(Ray64& R, const so_scene& S, bool emi
 // projection, controller, termination.  Returns 1 when the ray is finished.  Without `emit` only the
 // geometry advances (the ray's transmittance stays 1, so it ends only by capture, escape or the step
 // limit, never earlier than with emission).
-template <int VAR>
-__device__ __forceinline__ int ray_commit(Ray64& R, const so_scene& S, const so_frame& F, const float* field,
+template <int VAR, class Scene>
+__device__ __forceinline__ int ray_commit(Ray64& R, const Scene& H, const so_scene& S, const so_frame& F,
+                                          const float* field,
                                           const TorusParams& tp, double delta, bool emit,
                                           const double* yn, const double* k7, double hc, double err, int* fate,
                                           double* th, double* ph) {
-    if (VAR == VAR_RADIO && S.flow_on && yn[0] < S.r_flow_max) {
+    if (VAR == VAR_RADIO && H.flow_on && yn[0] < H.r_flow_max) {
         ++R.nflow;
         if (emit) {
             double dI, dtau;
@@ -250,11 +258,11 @@ __device__ __forceinline__ int ray_commit(Ray64& R, const so_scene& S, const so_
     }
     project_radial_fast(R.c, R.y, R.k1);
     R.h = accept_step_fast(hc, err);
-    if (R.y[0] < S.r_stop) {
+    if (R.y[0] < H.r_stop) {
         *fate = -1;
         return 1;
     }
-    if (R.y[0] > S.r_escape && R.y[1] > 0.0) {
+    if (R.y[0] > H.r_escape && R.y[1] > 0.0) {
         *fate = 1;
         escape_angles(R.y, R.k1, th, ph);
         return 1;
@@ -387,22 +395,31 @@ __device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
 
 }  // namespace
 
-// Register budget: three 128-thread CTAs per SM (at most 170 registers).  Measured on the B200
-// against the compiler's free choice (194 registers, two CTAs): the plain FP64 synchrotron frame
-// runs 1.29x faster with a few spilled registers and 50 % more warps.
-// DEFER (deferred FP64 passes, radio only): 0 = emission in the tracer, 1 = recording pass (geometry
-// only: no emission code), 2 = replay pass, 3 = recording pass of a ray list (also records each
-// step's crossings and writes the rays' outputs without emission).  Both passes run four CTAs per
-// SM (128 registers): measured on the 1024^2 synchrotron frame, the replay pass takes 178 ms there against 205 ms at
-// three CTAs (168 registers, fewer spills); the recording pass 78 ms, against 84 ms at five CTAs
-// (96 registers) and 88 ms at six (80), whose spills cost more than the warps gain (the reference
-// flow frame: 80, 89 and 100 ms).
-template <int VAR, bool EMIT32, int DEFER>
-__global__ void __launch_bounds__(128, DEFER >= 1 ? 4 : 3) k_trace64(const TraceLaunch L) {
+// DEFER (deferred FP64 passes, radio only): 0 = emission in the tracer; 1 = recording pass on the torus
+// with its modes (geometry only: no emission code; records hold the advected azimuth), 4 = recording
+// pass of the flow form; 3 and 5 = the same two for a ray list (also record each step's crossings and
+// write the rays' outputs without emission); 2 = replay pass.
+// HOT: one scene, whose values come from the launch descriptor (constant-bank operands) and not from the
+// ray's scene in memory; not for the radio kernels with the emission inside, where it made no difference.  TIME: the coordinate time is integrated (vacuum rays, and disks without turbulence,
+// never read it).
+//
+// Register budget.  An SM's scheduler holds 3 warps at 168 registers, 4 at 128, so 128-thread CTAs come
+// three or four to an SM; which is better is what the extra warp hides against the spills it costs.
+// Measured (recording pass, three against four): the reference flow 501 x 375 frame 39.0 against 47.8 ms,
+// the 262,144-ray list 10.9 against 11.0, the 1024^2 torus frame 50.4 against 46.2 (the logarithm and
+// roots of the torus phase run on a third of the lanes, which the fourth warp hides); thin disk
+// 1280 x 720 x 2 19.9 against 21.9; 65,536 vacuum rays 2.8 against 3.1; five (96 registers) lose everywhere.
+constexpr int tracer_ctas(int var, int defer) {
+    return defer == 1 || defer == 2 || defer == 3 || var == VAR_DISK ? 4 : 3;
+}
+template <int VAR, bool EMIT32, int DEFER, bool HOT, bool TIME>
+__global__ void __launch_bounds__(128, tracer_ctas(VAR, DEFER)) k_trace64(const __grid_constant__ TraceLaunch L) {
     extern __shared__ double smem[];
-    constexpr int defer = (VAR == VAR_RADIO && !EMIT32) ? (DEFER == 3 ? 1 : DEFER) : 0;
+    constexpr int defer = (VAR == VAR_RADIO && !EMIT32) ? (DEFER >= 3 ? 1 : DEFER) : 0;
     constexpr bool emit = defer != 1;
-    constexpr bool list_rec = defer == 1 && DEFER == 3;  // the recording pass of a ray list
+    constexpr bool list_rec = defer == 1 && (DEFER == 3 || DEFER == 5);  // the recording pass of a ray list
+    constexpr bool hot = HOT && (VAR != VAR_RADIO || defer == 1);
+    constexpr bool torus_rec = defer == 1 && (DEFER == 1 || DEFER == 3);
     // the replay pass behind the deferred emission runs only when the recording pass left samples
     // without records (the same value for every thread: the whole grid returns)
     if (defer == 2 && L.replay_if_short && *(volatile unsigned long long*)&L.rec64_ctl[1] == 0ull) return;
@@ -479,8 +496,10 @@ __global__ void __launch_bounds__(128, DEFER >= 1 ? 4 : 3) k_trace64(const Trace
     // grabbing lanes) and works through them before grabbing again.
     const int qchunk = L.queue_chunk > 1 ? L.queue_chunk : 1;
     int chunk_left = 0;
+    const bool worker = (lane & (stride - 1)) == 0;
     for (;;) {
-        const bool need = !active && !exhausted && (lane & (stride - 1)) == 0;
+        if (__any_sync(FULL, !active && !exhausted && worker)) {
+        const bool need = !active && !exhausted && worker;
         const bool grab = need && chunk_left == 0;
         const unsigned m = __ballot_sync(FULL, grab);
         unsigned long long j = (unsigned long long)(job - L.job0) + 1;  // the next job of the lane's grab
@@ -527,22 +546,23 @@ __global__ void __launch_bounds__(128, DEFER >= 1 ? 4 : 3) k_trace64(const Trace
             }
         }
         if (__all_sync(FULL, !active)) break;
+        }
         // ---- first half: the attempt (active lanes) ------------------------------------------
         int fate = 0, stage = ST_REJECTED;
         double yn[6], k7[6], hc = 0.0, err = 0.0;
         bool want = false;
         double TX = 0.0, TY = 0.0, TZ = 0.0;  // the sum's position (recording / replay pass: TX = azimuth)
+        auto& H = step_scene<hot>(L, S);
         if (active) {
-            stage = ray_attempt<VAR>(R, *S, emit, yn, k7, &hc, &err, &fate, rec ? cr : nullptr, cg);
-            if (VAR == VAR_RADIO && stage == ST_ACCEPTED && S->flow_on && yn[0] < S->r_flow_max) {
-                if (tp.n_modes > 0) {
-                    if (defer == 1 || (defer == 2 && !rinline))
-                        want = torus_phase(*S, tp, F->r, yn[0], yn[2], yn[4], yn[5], &TX);
-                    else
-                        want = torus_position(*S, tp, F->r, yn[0], yn[2], yn[4], yn[5], &TX, &TY, &TZ);
-                } else if (defer == 1) {
-                    // no turbulence sums: the torus without modes or the reference flow model
-                    want = tp.on ? torus_wants(*S, tp, yn[0], yn[2]) : flow_wants(*S, yn[0], yn[2]);
+            stage = ray_attempt<VAR, TIME>(R, H, *S, emit, yn, k7, &hc, &err, &fate, rec ? cr : nullptr, cg);
+            if (VAR == VAR_RADIO && stage == ST_ACCEPTED && H.flow_on && yn[0] < H.r_flow_max) {
+                if (defer == 1) {
+                    // the flow form has no turbulence sums: the torus without modes or the reference flow
+                    if (torus_rec) want = torus_phase(H, tp, hot ? L.hot.rcam : F->r, yn[0], yn[2], yn[4], yn[5], &TX);
+                    else want = tp.on ? torus_wants(H, tp, yn[0], yn[2]) : flow_wants(H, yn[0], yn[2]);
+                } else if (tp.n_modes > 0) {
+                    if (defer == 2 && !rinline) want = torus_phase(H, tp, hot ? L.hot.rcam : F->r, yn[0], yn[2], yn[4], yn[5], &TX);
+                    else want = torus_position(H, tp, hot ? L.hot.rcam : F->r, yn[0], yn[2], yn[4], yn[5], &TX, &TY, &TZ);
                 }
             }
         }
@@ -585,10 +605,10 @@ __global__ void __launch_bounds__(128, DEFER >= 1 ? 4 : 3) k_trace64(const Trace
                     double* slot = L.rec64 + (long long)L.rec64_w * ((long long)rseg * REC_SEG + rcnt);
                     slot[0] = yn[0];
                     slot[1] = yn[2];
-                    slot[2] = tp.n_modes > 0 ? TX : yn[4];
+                    slot[2] = torus_rec ? TX : yn[4];
                     slot[3] = hc;
                     slot[4] = __longlong_as_double((long long)tag);
-                    if (tp.n_modes <= 0) slot[5] = yn[5];
+                    if (!torus_rec) slot[5] = yn[5];
                     if (list_rec) slot[L.rec64_w - 1] = (double)R.ncross;
                     ++rcnt;
                     ++rtot;
@@ -619,7 +639,7 @@ __global__ void __launch_bounds__(128, DEFER >= 1 ? 4 : 3) k_trace64(const Trace
         if (!active || stage == ST_REJECTED) continue;
         double th = 0.0, ph = 0.0;
         if (stage == ST_ACCEPTED &&
-            !ray_commit<VAR>(R, *S, *F, L.turb_field, tp, delta, emit, yn, k7, hc, err, &fate, &th, &ph))
+            !ray_commit<VAR>(R, H, *S, *F, L.turb_field, tp, delta, emit, yn, k7, hc, err, &fate, &th, &ph))
             continue;
         // sample finished
         if (defer == 1) {
@@ -1133,14 +1153,25 @@ cudaError_t launch_trace64(const TraceLaunch& L, int variant, int num_sms, cudaS
         return cudaGetLastError();
     };
     switch (variant) {
-        case VAR_VACUUM: return go(k_trace64<VAR_VACUUM, false, 0>);
-        case VAR_DISK: return go(k_trace64<VAR_DISK, false, 0>);
+        case VAR_VACUUM:
+            return L.hot_ok ? go(k_trace64<VAR_VACUUM, false, 0, true, false>)
+                            : go(k_trace64<VAR_VACUUM, false, 0, false, false>);
+        case VAR_DISK:
+            if (L.disk_time || !L.hot_ok) return go(k_trace64<VAR_DISK, false, 0, false, true>);
+            return go(k_trace64<VAR_DISK, false, 0, true, false>);
         default:
-            if (emit32) return go(k_trace64<VAR_RADIO, true, 0>);
+            if (emit32) return go(k_trace64<VAR_RADIO, true, 0, false, true>);
+            if (L.defer64 == 1 && L.kind == RAYS_LIST)  // always one scene's (run_tracer)
+                return torus ? go(k_trace64<VAR_RADIO, false, 3, true, true>)
+                             : go(k_trace64<VAR_RADIO, false, 5, true, true>);
+            if (L.defer64 == 1 && torus)
+                return L.hot_ok ? go(k_trace64<VAR_RADIO, false, 1, true, true>)
+                                : go(k_trace64<VAR_RADIO, false, 1, false, true>);
             if (L.defer64 == 1)
-                return L.kind == RAYS_LIST ? go(k_trace64<VAR_RADIO, false, 3>) : go(k_trace64<VAR_RADIO, false, 1>);
-            if (L.defer64 == 2) return go(k_trace64<VAR_RADIO, false, 2>);
-            return go(k_trace64<VAR_RADIO, false, 0>);
+                return L.hot_ok ? go(k_trace64<VAR_RADIO, false, 4, true, true>)
+                                : go(k_trace64<VAR_RADIO, false, 4, false, true>);
+            if (L.defer64 == 2) return go(k_trace64<VAR_RADIO, false, 2, false, true>);
+            return go(k_trace64<VAR_RADIO, false, 0, false, true>);
     }
 }
 

@@ -225,15 +225,16 @@ __device__ __forceinline__ bool profile_wants(double u2, double w2) { return !(u
 // Where the torus turbulence is needed for a flow step at (r, u, phi, t): false when flow_step
 // returns before using it (only those flow steps can change the transfer); else the advected
 // azimuth phc of the sum's position.
-__device__ __forceinline__ bool torus_phase(const so_scene& S, const TorusParams& tp, double rcam, double r, double u,
+template <class Scene>
+__device__ __forceinline__ bool torus_phase(const Scene& H, const TorusParams& tp, double rcam, double r, double u,
                                             double phi, double t, double* phc) {
     if (!tp.on || tp.n_modes <= 0) return false;
     double s2 = fmax(fma(-u, u, 1.0), 1e-12), s = fast_sqrt(s2);
     double R = r * s;
-    if (r > S.r_flow_max || R < 1e-3) return false;
+    if (r > H.r_flow_max || R < 1e-3) return false;
     if (!profile_wants(u * u, tp.h_sph * tp.h_sph)) return false;
-    const double Rk = fmax(R, S.r_isco);
-    double Omf = S.flow_kep * fast_rcp(fma(Rk, fast_sqrt(Rk), S.a));
+    const double Rk = fmax(R, H.r_isco);
+    double Omf = H.flow_kep * fast_rcp(fma(Rk, fast_sqrt(Rk), H.a));
     *phc = phi - Omf * (t + (rcam - r + 2.0 * log(fast_div(rcam, r))));
     return true;
 }
@@ -247,10 +248,11 @@ __device__ __forceinline__ void torus_xyz(double r, double u, double phc, double
     *Y = R * sp;
     *Z = r * u;
 }
-__device__ __forceinline__ bool torus_position(const so_scene& S, const TorusParams& tp, double rcam, double r,
-                                               double u, double phi, double t, double* X, double* Y, double* Z) {
+template <class Scene>
+__device__ __forceinline__ bool torus_position(const Scene& H, const TorusParams& tp, double rcam, double r, double u,
+                                               double phi, double t, double* X, double* Y, double* Z) {
     double phc;
-    if (!torus_phase(S, tp, rcam, r, u, phi, t, &phc)) return false;
+    if (!torus_phase(H, tp, rcam, r, u, phi, t, &phc)) return false;
     torus_xyz(r, u, phc, X, Y, Z);
     return true;
 }
@@ -297,16 +299,18 @@ __device__ __forceinline__ float baked_sample(const so_scene& S, const float* fi
 
 // Whether flow_step on the reference flow model (no torus) can change the transfer at (r, u): its
 // first two returns.  A step for which this is false emits nothing and transmits exactly 1.
-__device__ __forceinline__ bool flow_wants(const so_scene& S, double r, double u) {
+template <class Scene>
+__device__ __forceinline__ bool flow_wants(const Scene& H, double r, double u) {
     const double s2 = fmax(fma(-u, u, 1.0), 1e-12);
     // R^2 = r^2 sin^2, and zh = z / (h R) = u / (h sin)
-    return !(r > S.r_flow_max) && !(r * r * s2 < 0.999999999e-6) && profile_wants(u * u, S.h_r * S.h_r * s2);
+    return !(r > H.r_flow_max) && !(r * r * s2 < 0.999999999e-6) && profile_wants(u * u, H.h_r * H.h_r * s2);
 }
 
 // The same for the torus plasma (flow_step's torus branch: zh = u / h_sph).
-__device__ __forceinline__ bool torus_wants(const so_scene& S, const TorusParams& tp, double r, double u) {
+template <class Scene>
+__device__ __forceinline__ bool torus_wants(const Scene& H, const TorusParams& tp, double r, double u) {
     const double s2 = fmax(fma(-u, u, 1.0), 1e-12);
-    return !(r > S.r_flow_max) && !(r * r * s2 < 0.999999999e-6) && profile_wants(u * u, tp.h_sph * tp.h_sph);
+    return !(r > H.r_flow_max) && !(r * r * s2 < 0.999999999e-6) && profile_wants(u * u, tp.h_sph * tp.h_sph);
 }
 
 // flow_step with the torus turbulence sum `delta` at this point already evaluated (torus_position).

@@ -74,7 +74,10 @@ SO_HD double sin_of(double u) {
 }
 
 // rhs() with the two quotients above.  A Delta or sin^2 outside the normal range makes d[4] infinite
-// or NaN.
+// or NaN.  1 - u^2 in one rounding is at most 0 or at least 2^-53, so the sign of its high word
+// is the test against 1e-300 (a NaN goes through to d[4]).  Without TIME the coordinate time is left out (d[5] = 0): nothing depends
+// on it but the emission.
+template <bool TIME = true>
 SO_HD void rhs_fast(const RayC& c, const double* y, double* d) {
     double r = y[0], u = y[2];
     double r2 = r * r;
@@ -86,47 +89,65 @@ SO_HD void rhs_fast(const RayC& c, const double* y, double* d) {
     double u2 = u * u;
     d[3] = u * fma(c.A2, fma(-2.0, u2, 1.0), -c.Q3);
     double s2 = 1.0 - u2;
-    s2 = s2 > 1e-300 ? s2 : 1e-300;
+    s2 = (int)(dbits(s2) >> 32) > 0 ? s2 : 1e-300;
     double iD = fast_rcp(Delta);
     d[4] = c.a - fma(c.a * P, iD, fast_div(c.lam, s2));
-    d[5] = -fma((r2 + c.A2) * P, iD, c.a * fma(-c.a, s2, c.lam));
+    d[5] = TIME ? -fma((r2 + c.A2) * P, iD, c.a * fma(-c.a, s2, c.lam)) : 0.0;
 }
+
+// The Dormand-Prince coefficients as constant-bank operands: as literals each use costs two moves (a
+// 64-bit immediate does not fit an instruction).
+struct Tableau {
+    double a21, a31, a32, a41, a42, a43, a51, a52, a53, a54, a61, a62, a63, a64, a65, b1, b3, b4, b5, b6, e1, e3, e4, e5, e6, e7;
+};
+#define SO_TABLEAU_VALUES {A21, A31, A32, A41, A42, A43, A51, A52, A53, A54, A61, A62, A63, A64, A65, B1, B3, B4, B5, B6, E1, E3, E4, E5, E6, E7}
+#if defined(__CUDACC__)
+static __constant__ Tableau dp_tableau = SO_TABLEAU_VALUES;
+#endif
+#if defined(__CUDA_ARCH__)
+#define SO_TABLEAU(T) const Tableau& T = dp_tableau
+#else
+#define SO_TABLEAU(T) static const Tableau T = SO_TABLEAU_VALUES
+#endif
 
 // dp54() in the same arithmetic; *ok says whether every operand stayed in range (else the result is
 // not to be used).  The error norm is the largest of five quotients |e_i| / sc_i.  Rounding is
 // monotone, so it is the rounded quotient of the largest ratio, found by comparing products; the two
 // constant denominators tol and 4 tol share one candidate (the factor 4 is exact).  A NaN candidate
 // is passed over, as fmax does.  Four divisions fewer.
+template <bool TIME = true>
 SO_HD double dp54_fast(const RayC& c, const double* y, const double* k1, double h, double tol, double* yo,
                        double* k7, bool* ok) {
+    SO_TABLEAU(T);
     double k2[6], k3[6], k4[6], k5[6], k6[6], t[6];
     t[4] = y[4];
     t[5] = y[5];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) t[i] = fma(h, A21 * k1[i], y[i]);
-    rhs_fast(c, t, k2);  // (the phi and t components of k2 enter nothing)
+    for (int i = 0; i < 4; ++i) t[i] = fma(h, T.a21 * k1[i], y[i]);
+    rhs_fast<TIME>(c, t, k2);  // (the phi and t components of k2 enter nothing)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) t[i] = fma(h, fma(A32, k2[i], A31 * k1[i]), y[i]);
-    rhs_fast(c, t, k3);
+    for (int i = 0; i < 4; ++i) t[i] = fma(h, fma(T.a32, k2[i], T.a31 * k1[i]), y[i]);
+    rhs_fast<TIME>(c, t, k3);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) t[i] = fma(h, fma(A43, k3[i], fma(A42, k2[i], A41 * k1[i])), y[i]);
-    rhs_fast(c, t, k4);
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-        t[i] = fma(h, fma(A54, k4[i], fma(A53, k3[i], fma(A52, k2[i], A51 * k1[i]))), y[i]);
-    rhs_fast(c, t, k5);
+    for (int i = 0; i < 4; ++i) t[i] = fma(h, fma(T.a43, k3[i], fma(T.a42, k2[i], T.a41 * k1[i])), y[i]);
+    rhs_fast<TIME>(c, t, k4);
 #pragma unroll
     for (int i = 0; i < 4; ++i)
-        t[i] = fma(h, fma(A65, k5[i], fma(A64, k4[i], fma(A63, k3[i], fma(A62, k2[i], A61 * k1[i])))), y[i]);
-    rhs_fast(c, t, k6);
+        t[i] = fma(h, fma(T.a54, k4[i], fma(T.a53, k3[i], fma(T.a52, k2[i], T.a51 * k1[i]))), y[i]);
+    rhs_fast<TIME>(c, t, k5);
 #pragma unroll
-    for (int i = 0; i < 6; ++i)
-        yo[i] = fma(h, fma(B6, k6[i], fma(B5, k5[i], fma(B4, k4[i], fma(B3, k3[i], B1 * k1[i])))), y[i]);
-    rhs_fast(c, yo, k7);
+    for (int i = 0; i < 4; ++i)
+        t[i] = fma(h, fma(T.a65, k5[i], fma(T.a64, k4[i], fma(T.a63, k3[i], fma(T.a62, k2[i], T.a61 * k1[i])))), y[i]);
+    rhs_fast<TIME>(c, t, k6);
+#pragma unroll
+    for (int i = 0; i < (TIME ? 6 : 5); ++i)
+        yo[i] = fma(h, fma(T.b6, k6[i], fma(T.b5, k5[i], fma(T.b4, k4[i], fma(T.b3, k3[i], T.b1 * k1[i])))), y[i]);
+    if (!TIME) yo[5] = y[5];
+    rhs_fast<TIME>(c, yo, k7);
     double e[5];
 #pragma unroll
     for (int i = 0; i < 5; ++i)
-        e[i] = fabs(h * fma(E7, k7[i], fma(E6, k6[i], fma(E5, k5[i], fma(E4, k4[i], fma(E3, k3[i], E1 * k1[i]))))));
+        e[i] = fabs(h * fma(T.e7, k7[i], fma(T.e6, k6[i], fma(T.e5, k5[i], fma(T.e4, k4[i], fma(T.e3, k3[i], T.e1 * k1[i]))))));
     const double a0 = fabs(y[0]), b0 = fabs(yo[0]), a1 = fabs(y[1]), b1 = fabs(yo[1]);
     const double a3 = fabs(y[3]), b3 = fabs(yo[3]), rr = y[0] * y[0];
     double m1 = b1 > a1 ? b1 : a1;
@@ -160,10 +181,11 @@ static __device__ __noinline__ double dp54_again(const RayC* c, const double* yk
     return dp54(*c, yk, yk + 6, h, tol, yo, yo + 6);
 }
 // dp54() through the fast form: the same steps and the same error.
+template <bool TIME>
 __device__ __forceinline__ double dp54_attempt(const RayC& c, const double* y, const double* k1, double h, double tol,
                                                double* yo, double* k7) {
     bool ok;
-    double err = dp54_fast(c, y, k1, h, tol, yo, k7, &ok);
+    double err = dp54_fast<TIME>(c, y, k1, h, tol, yo, k7, &ok);
     if (!ok) {
         double yk[12], out[12];
         const RayC cc = c;

@@ -102,7 +102,18 @@ struct LumScratch {
 cudaError_t post_luminance(const float4* img, long long n, int radio, float hide, double percentile,
                            const LumScratch& s, cudaStream_t st);
 
+// The scene values that every step of the tracer reads.  A launch on one scene carries them in its
+// descriptor, so that they are constant-bank operands and not loads.
+struct HotScene {
+    double tol, step_frac, r_flow_max, r_stop, r_escape;
+    double a, r_isco, flow_kep, h_r, rcam;
+    int max_steps, flow_on, disk_on;
+};
+
 struct TraceLaunch {
+    HotScene hot;             // scene 0 and frame 0, for launches with hot_ok (one scene, one frame)
+    int hot_ok;
+    int disk_time;            // disk variant: the shading reads the coordinate time (disk turbulence)
     const so_scene* scenes;   // device array, indexed by frame_scene[f]
     const so_frame* frames;   // device array
     const int* frame_scene;   // device array

@@ -57,6 +57,7 @@ struct so_renderer {
     int device = 0, num_sms = 148;
     cudaStream_t st = nullptr;
     so_scene S{};            // host copy, table pointers = device tables
+    so_frame F{};            // host copy of the frame last uploaded to d_frame
     so_settings rs{};
     float *d_disk = nullptr, *d_k2 = nullptr, *d_bb = nullptr;
     so_scene* d_scene = nullptr;
@@ -374,7 +375,15 @@ int bake_turbulence(so_renderer* r, TraceLaunch& L) {
     return SO_OK;
 }
 
-// Fills the plasma / precision part of a launch descriptor.
+// Upload of the frame that the next launches trace.
+int upload_frame(so_renderer* r, const so_frame& f) {
+    r->F = f;
+    SO_CK(r, cudaMemcpyAsync(r->d_frame, &f, sizeof f, cudaMemcpyHostToDevice, r->st));
+    return SO_OK;
+}
+
+// Fills the scene and plasma / precision part of a launch descriptor (one scene: that of d_scene, with
+// the frame of upload_frame).
 void launch_common(so_renderer* r, TraceLaunch& L) {
     std::memset(&L, 0, sizeof L);
     L.scenes = r->d_scene;
@@ -382,6 +391,11 @@ void launch_common(so_renderer* r, TraceLaunch& L) {
     L.frame_scene = r->d_frame_scene;
     L.nframes = 1;
     L.counters = r->d_cnt;
+    const so_scene& S = r->S;
+    L.hot = {S.tol, S.step_frac, S.r_flow_max, S.r_stop, S.r_escape, S.a, S.r_isco, S.flow_kep, S.h_r, r->F.r,
+             S.max_steps, S.flow_on, S.disk_on};
+    L.hot_ok = 1;
+    L.disk_time = S.disk_turb_amp > 0.f;
     const so_plasma& p = r->plasma;
     L.torus = p.model == SO_PLASMA_TORUS;
     L.n_modes = L.torus ? p.n_modes : 0;
@@ -1000,7 +1014,7 @@ int trace_frame(so_renderer* r, const so_frame& f, bool adaptive, so_stats* stat
                 if (e[i]) cudaEventDestroy(e[i]);
         }
     } guard{ev};
-    SO_CK(r, cudaMemcpyAsync(r->d_frame, &f, sizeof f, cudaMemcpyHostToDevice, r->st));
+    if (int frc = upload_frame(r, f)) return frc;
     SO_CK(r, cudaMemsetAsync(r->d_cnt, 0, sizeof(Counters), r->st));
     r->list_rays = 0;
     const long long n = (long long)f.W * f.H;
@@ -1229,7 +1243,7 @@ int rend_band_table(so_renderer* r, double th, const float** d_band, int* n) {
 }
 
 int rend_upload_frame(so_renderer* r, const so_frame& f, const so_frame** d_frame) {
-    SO_CK(r, cudaMemcpyAsync(r->d_frame, &f, sizeof(so_frame), cudaMemcpyHostToDevice, r->st));
+    if (int rc = upload_frame(r, f)) return rc;
     *d_frame = r->d_frame;
     return SO_OK;
 }
@@ -1279,6 +1293,8 @@ int rend_trace_list_frames(so_renderer* r, int n, const double* d_x, const doubl
     L.frame_scene = d_frame_scene;
     L.nframes = nframes;
     L.list_frames = nframes;
+    L.hot_ok = 0;
+    L.disk_time = 1;
     L.kind = RAYS_LIST;
     L.nrays = n;
     L.x = d_x;
@@ -1462,7 +1478,7 @@ int so_radio_flux(so_renderer* r, const so_frame* f_in, int n, double pix_sr, do
 
 static int trace_rays_impl(so_renderer* r, const so_frame* f, int n, const double* d_x, const double* d_y,
                            const so_rays_out& d_out) {
-    SO_CK(r, cudaMemcpyAsync(r->d_frame, f, sizeof(so_frame), cudaMemcpyHostToDevice, r->st));
+    if (int frc = upload_frame(r, *f)) return frc;
     SO_CK(r, cudaMemsetAsync(r->d_cnt, 0, sizeof(Counters), r->st));
     r->list_rays = 0;
     TraceLaunch L;
@@ -1793,6 +1809,8 @@ void batch_launch_desc(so_batch* b, float* d_px, TraceLaunch& L) {
     so_renderer* r = b->r;
     launch_common(r, L);
     L.scenes = b->d_scenes;
+    L.hot_ok = 0;
+    L.disk_time = 1;
     L.frames = b->d_frames;
     L.frame_scene = b->d_frame_scene;
     L.nframes = b->nframes;
