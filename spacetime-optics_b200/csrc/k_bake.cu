@@ -40,11 +40,11 @@ struct RunTable {
 
 // Gradient of lattice corner hash h: grad3's two signed components (so_emission.cuh) as a vector.
 __device__ __forceinline__ void corner_grad(uint32_t h, float* g) {
-    const uint32_t c = h % 12u;
-    const float su = (c & 1u) ? -1.f : 1.f, sv = (c & 2u) ? -1.f : 1.f;
-    g[0] = c < 8u ? su : 0.f;
-    g[1] = c < 4u ? sv : (c < 8u ? 0.f : su);
-    g[2] = c < 4u ? 0.f : sv;
+    const uint32_t third = (h >> 2) * 0x55555556u;
+    const float su = (h & 1u) ? -1.f : 1.f, sv = (h & 2u) ? -1.f : 1.f;
+    g[0] = third < 0xAAAAAAAAu ? su : 0.f;
+    g[1] = third < 0x55555555u ? sv : (third < 0xAAAAAAAAu ? 0.f : su);
+    g[2] = third < 0x55555555u ? 0.f : sv;
 }
 
 // Hash of the table's runs [0, n): lane by lane, the corners in gnoise's nesting (z, then y, then x).

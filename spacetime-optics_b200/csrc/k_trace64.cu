@@ -923,7 +923,7 @@ cudaError_t launch_turb32_rec64(const TraceLaunch& L, const TurbModes& M, int nu
 // the flow records' form (phi, t) and reads neither; the reference flow model reads its phi and t
 // and fetches the frame's turbulence as the tracer does.  Left to the replay pass when a sample ran
 // out of segments.
-__global__ void __launch_bounds__(256) k_emit64_records(const TraceLaunch L) {
+__global__ void __launch_bounds__(256, 3) k_emit64_records(const TraceLaunch L) {
     if (*(volatile unsigned long long*)&L.rec64_ctl[1] != 0ull) return;
     unsigned long long used = *(volatile unsigned long long*)&L.rec64_ctl[0];
     if (used > (unsigned long long)L.seg_cap64) used = (unsigned long long)L.seg_cap64;
@@ -987,30 +987,42 @@ __global__ void __launch_bounds__(128) k_transfer64(const TraceLaunch L) {
             double trans = 1.0;
             int fate = e.fate, natt = e.natt, nacc = e.nacc, nflow = e.nflow, ncut = -1;
             long long seg = L.job_head64[sid];
-            for (int i = 0; i < e.nrec; ++i) {
+            // four records of a segment are loaded ahead of the chain that applies them
+            for (int i = 0; i < e.nrec && ncut == -1; i += 4) {
                 const int k = i % REC_SEG;
                 if (k == 0 && i > 0) seg = (long long)L.seg_next64[seg];
                 if (seg < 0 || seg >= L.seg_cap64) {  // never with a complete chain; visible, not a stray read
                     acc[0] = __int_as_float(0x7fc00000);
                     break;
                 }
+                const int m = min(4, e.nrec - i);
                 const double* rec = L.rec64 + (long long)L.rec64_w * (seg * REC_SEG + k);
-                const double dI = rec[0], ex = rec[1];
-                const unsigned long long tag = (unsigned long long)__double_as_longlong(rec[4]);
-                const float cc = (float)(trans * dI);
-                const int b = (int)(tag & 3ull);
-                acc[0] += cc;
-                if (b == 1) acc[1] += cc;
-                else if (b == 2) acc[2] += cc;
-                else if (b == 3) acc[3] += cc;
-                trans *= ex;
-                if (trans < 1e-5) {
-                    fate = -1;
-                    natt = (int)((tag >> 2) & cmask);
-                    nacc = (int)((tag >> (2 + REC64_COUNT_BITS)) & cmask);
-                    nflow = (int)((tag >> (2 + 2 * REC64_COUNT_BITS)) & cmask);
-                    if (L.kind == RAYS_LIST) ncut = (int)rec[L.rec64_w - 1];
-                    break;
+                double dI[4], ex[4], tg[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const double* rc = rec + (c < m ? L.rec64_w * c : 0);
+                    dI[c] = rc[0];
+                    ex[c] = rc[1];
+                    tg[c] = rc[4];
+                }
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    if (c >= m || ncut != -1) continue;
+                    const unsigned long long tag = (unsigned long long)__double_as_longlong(tg[c]);
+                    const float cc = (float)(trans * dI[c]);
+                    const int b = (int)(tag & 3ull);
+                    acc[0] += cc;
+                    if (b == 1) acc[1] += cc;
+                    else if (b == 2) acc[2] += cc;
+                    else if (b == 3) acc[3] += cc;
+                    trans *= ex[c];
+                    if (trans < 1e-5) {
+                        fate = -1;
+                        natt = (int)((tag >> 2) & cmask);
+                        nacc = (int)((tag >> (2 + REC64_COUNT_BITS)) & cmask);
+                        nflow = (int)((tag >> (2 + 2 * REC64_COUNT_BITS)) & cmask);
+                        ncut = L.kind == RAYS_LIST ? (int)rec[L.rec64_w * c + L.rec64_w - 1] : 0;
+                    }
                 }
             }
             n_att += (unsigned long long)natt;

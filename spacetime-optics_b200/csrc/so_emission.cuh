@@ -59,12 +59,16 @@ __device__ __forceinline__ void sample_point(int W, int H, int jitter, const so_
 // switch on a hash diverges in every warp): case g < 8 takes fx first, else fy; g < 4 takes fy
 // second, else fz; bit 0 of g negates the first term, bit 1 the second.  Same sums, bit for bit
 // (a - b is a + (-b) in IEEE arithmetic).
+//
+// The case is h mod 12 = 4 ((h >> 2) mod 3) + (h & 3), so the sign bits are h's own and the choice needs
+// only x mod 3 of the 30-bit x = h >> 2: with K = (2^32 + 2) / 3, the low word of x K is
+// 2^32 (x mod 3) / 3 + 2 x / 3, and 2 x / 3 < 2^32 / 6 cannot reach the next third.
 __device__ __forceinline__ float grad3(int ix, int iy, int iz, uint32_t seed, float fx, float fy, float fz) {
     uint32_t h = pcg((uint32_t)ix * 73856093u ^ pcg((uint32_t)iy * 19349663u ^ pcg((uint32_t)iz * 83492791u ^ seed)));
-    const uint32_t g = h % 12u;
-    const float u = g < 8u ? fx : fy;
-    const float v = g < 4u ? fy : fz;
-    return ((g & 1u) ? -u : u) + ((g & 2u) ? -v : v);
+    const uint32_t third = (h >> 2) * 0x55555556u;
+    const float u = third < 0xAAAAAAAAu ? fx : fy;
+    const float v = third < 0x55555555u ? fy : fz;
+    return ((h & 1u) ? -u : u) + ((h & 2u) ? -v : v);
 }
 static __device__ float gnoise(float x, float y, float z, uint32_t seed) {
     float fx = floorf(x), fy = floorf(y), fz = floorf(z);
@@ -87,6 +91,7 @@ static __device__ float gnoise(float x, float y, float z, uint32_t seed) {
 }
 static __device__ float fbm3(float x, float y, float z, int oct, uint32_t seed) {
     float s = 0.f, amp = 1.f, norm = 0.f;
+#pragma unroll 1  // eight inlined copies of gnoise (two generations, four octaves) overflow the instruction cache
     for (int i = 0; i < oct; ++i) {
         s += amp * gnoise(x, y, z, seed + 1013u * (uint32_t)i);
         norm += amp * amp;
@@ -128,6 +133,7 @@ static __device__ float sheared_noise(const so_scene& S, double R, double phi, d
     double k = floor(s);
     float f = (float)(s - k);
     float acc = 0.f;
+#pragma unroll 1
     for (int j = 0; j < 2; ++j) {
         double tb = (k + j) * P;
         double ph = phi - Om * (t - tb);
@@ -313,39 +319,63 @@ __device__ __forceinline__ bool torus_wants(const Scene& H, const TorusParams& t
     return !(r > H.r_flow_max) && !(r * r * s2 < 0.999999999e-6) && profile_wants(u * u, tp.h_sph * tp.h_sph);
 }
 
+// The arithmetic of flow_step: quotients and roots by the IEEE operators, or straight-line (so_fast64.cuh) with
+// a note of any operand outside [2^-495, 2^497), for which the step is taken again.
+struct IeeeOps {
+    __device__ __forceinline__ double div(double a, double b) { return a / b; }
+    __device__ __forceinline__ double near(double) { return 0.0; }
+    __device__ __forceinline__ double quot(double a, double b, double) { return a / b; }
+    __device__ __forceinline__ double sqrt(double x) { return ::sqrt(x); }
+};
+struct QuickOps {
+    unsigned bad = 0;
+    __device__ __forceinline__ void check(double x) { bad |= (unsigned)__double2hiint(x) - 0x21000000u >= 0x3e000000u; }
+    __device__ __forceinline__ double near(double b) {
+        check(b);
+        return near_rcp(b, seed_rcp(b));
+    }
+    __device__ __forceinline__ double quot(double a, double b, double y) { return round_quot(a, b, y); }
+    __device__ __forceinline__ double div(double a, double b) { return round_quot(a, b, near(b)); }
+    __device__ __forceinline__ double sqrt(double x) {
+        check(x);
+        return fast_sqrt(x);
+    }
+};
+
 // flow_step with the torus turbulence sum `delta` at this point already evaluated (torus_position).
 // With `field` (the frame's baked slices) the reference model's turbulence is sampled as
 // emission.cuh:112-124 does, else its sheared noise is evaluated in place (the turb_nt = 0 path).
-static __device__ void flow_step(const so_scene& S, const so_frame& F, const float* field, const TorusParams& tp,
+template <class M>
+__device__ __forceinline__ void flow_step_in(M& m, const so_scene& S, const so_frame& F, const float* field, const TorusParams& tp,
                                  double delta, double r, double u, double phi, double t, double lam, double Ecam,
                                  double h, double* dI, double* dtau) {
     *dI = 0.0;
     *dtau = 0.0;
     const double a = S.a;
-    double s2 = fmax(fma(-u, u, 1.0), 1e-12), s = sqrt(s2);
+    double s2 = fmax(fma(-u, u, 1.0), 1e-12), s = m.sqrt(s2);
     double R = r * s, z = r * u;
     if (r > S.r_flow_max || R < 1e-3) return;
     double ne, Th;
     if (tp.on) {
-        double zh = u / tp.h_sph;
+        double zh = m.div(u, tp.h_sph);
         double vert = exp(-0.5 * zh * zh);
         if (vert < 1e-7) return;
-        double lx = log(r / S.rh);
+        double lx = log(m.div(r, S.rh));
         ne = S.n0 * exp(-tp.ne_index * lx) * vert;
         if (tp.n_modes > 0) ne *= exp(delta - tp.half_var);
         Th = tp.theta_e0 * exp(-tp.te_index * lx);
     } else {
-        double zh = z / (S.h_r * R);
+        double zh = m.div(z, S.h_r * R);
         double vert = exp(-0.5 * zh * zh);
         if (vert < 1e-7) return;
         ne = S.n0 * exp(-S.n_index * log(r)) * vert;
         if (S.flow_turb_amp > 0.f) {
             if (baked_on(S, field)) {
                 // two slices around the retarded time t - t_ref(r), interpolated (emission.cuh:112-124)
-                const double tref = F.t - (F.r - r + 2.0 * log(F.r / r));
-                const float y = (float)((log(R) - S.turb_lr0) / (S.turb_lr1 - S.turb_lr0));
+                const double tref = F.t - (F.r - r + 2.0 * log(m.div(F.r, r)));
+                const float y = (float)m.div(log(R) - S.turb_lr0, (double)(S.turb_lr1 - S.turb_lr0));
                 const float x = (float)(phi * (0.5 / PI));
-                const float w = (float)(0.5 + 0.5 * (z / R) / S.turb_zmax);
+                const float w = (float)(0.5 + m.div(0.5 * m.div(z, R), (double)S.turb_zmax));
                 float sl = (float)((t - tref) - S.turb_d0) / S.turb_dd;
                 sl = fminf(fmaxf(sl, 0.f), (float)(TURB_NT - 1) - 1e-4f);
                 const int k = (int)sl;
@@ -364,42 +394,76 @@ static __device__ void flow_step(const so_scene& S, const so_frame& F, const flo
     ne *= 1.0 - exp(-(dr * dr) / 0.25);
     if (ne < 1e-30) return;
     if (!tp.on) Th = S.theta0 * exp(-S.theta_index * log(r));
-    double B = sqrt(8.0 * PI * ne * cgs::MP * cgs::C * cgs::C / (6.0 * r * S.beta_p));
+    double B = m.sqrt(m.div(8.0 * PI * ne * cgs::MP * cgs::C * cgs::C, 6.0 * r * S.beta_p));
     double r2 = r * r, a2 = a * a;
     double Sigma = fma(a2, u * u, r2), Delta = fma(r, r - 2.0, a2);
     double rpa = r2 + a2;
     double A = fma(rpa, rpa, -(a2 * Delta * s2));
-    double g_tt = -(1.0 - 2.0 * r / Sigma), g_tph = -2.0 * a * r * s2 / Sigma, g_phph = A * s2 / Sigma;
-    double omz = 2.0 * a * r / A;
-    double Om = S.flow_kep * keplerian_omega(a, fmax(R, S.r_isco));
-    double vmax = sqrt(Sigma * Delta / A) / sqrt(g_phph) * 0.999;
+    const double ySig = m.near(Sigma);
+    double g_tt = -(1.0 - m.quot(2.0 * r, Sigma, ySig)), g_tph = m.quot(-2.0 * a * r * s2, Sigma, ySig),
+           g_phph = m.quot(A * s2, Sigma, ySig);
+    const double yA = m.near(A);
+    double omz = m.quot(2.0 * a * r, A, yA);
+    const double Rk = fmax(R, S.r_isco);
+    double Om = S.flow_kep * m.div(1.0, fma(Rk, m.sqrt(Rk), a));
+    double vmax = m.div(m.sqrt(m.quot(Sigma * Delta, A, yA)), m.sqrt(g_phph)) * 0.999;
     Om = omz + fmax(-vmax, fmin(vmax, Om - omz));
     double norm = -fma(g_phph * Om, Om, fma(2.0 * g_tph, Om, g_tt));
     if (norm <= 0.0) return;
-    double ut = 1.0 / sqrt(norm);
+    double ut = m.div(1.0, m.sqrt(norm));
     double kdotu = ut * fma(-Om, lam, 1.0);
     double nu_f = S.nu_obs * Ecam * kdotu;
-    double g = S.nu_obs / nu_f;
+    double g = m.div(S.nu_obs, nu_f);
     double u_ph = ut * fma(g_phph, Om, g_tph);
     double kb = fma(-kdotu, u_ph, lam);
     double bb = fma(u_ph, u_ph, g_phph);
-    double cosb = kb / (kdotu * sqrt(bb));
-    double sinb = sqrt(fmax(fma(-cosb, cosb, 1.0), 1e-6));
-    double nuc = cgs::QE * B / (2.0 * PI * cgs::ME * cgs::C);
+    double cosb = m.div(kb, kdotu * m.sqrt(bb));
+    double sinb = m.sqrt(fmax(fma(-cosb, cosb, 1.0), 1e-6));
+    constexpr double kMec = 2.0 * PI * cgs::ME * cgs::C, kC2 = cgs::C * cgs::C;
+    double nuc = m.quot(cgs::QE * B, kMec, 1.0 / kMec);
     double nus = 2.0 / 9.0 * nuc * Th * Th * sinb;
-    double Xs = nu_f / nus;
+    double Xs = m.div(nu_f, nus);
     double x3 = cbrt(Xs);
     double k2 = exp((double)table_lerp(S.k2_lntab, S.k2_n, S.k2_l0, S.k2_dl, (float)log(Th)));
-    double brk = fma(1.887748625363387, sqrt(x3), sqrt(Xs));
-    double j = ne * 1.4142135623730951 * PI * cgs::QE * cgs::QE * nus / (3.0 * k2 * cgs::C) * brk * brk * exp(-x3);
-    double Te = Th * cgs::ME * cgs::C * cgs::C / cgs::KB;
-    double hnu = cgs::H * nu_f / (cgs::KB * Te);
-    double Bnu = 2.0 * cgs::H * nu_f * nu_f * nu_f / (cgs::C * cgs::C) / expm1(hnu);
-    double alpha = j / Bnu;
+    double brk = fma(1.887748625363387, m.sqrt(x3), m.sqrt(Xs));
+    double j = m.div(ne * 1.4142135623730951 * PI * cgs::QE * cgs::QE * nus, 3.0 * k2 * cgs::C) * brk * brk * exp(-x3);
+    double Te = m.quot(Th * cgs::ME * cgs::C * cgs::C, cgs::KB, 1.0 / cgs::KB);
+    double hnu = m.div(cgs::H * nu_f, cgs::KB * Te);
+    double Bnu = m.div(m.quot(2.0 * cgs::H * nu_f * nu_f * nu_f, kC2, 1.0 / kC2), expm1(hnu));
+    double alpha = m.div(j, Bnu);
     double dl = kdotu * Sigma * h * S.rg_cm;
     double tau = alpha * dl;
     *dtau = tau;
     *dI = g * g * g * Bnu * (-expm1(-tau));
+}
+
+
+static __device__ __noinline__ void flow_step_again(const so_scene& S, const so_frame& F, const float* field,
+                                                    const TorusParams& tp, double delta, double r, double u, double phi,
+                                                    double t, double lam, double Ecam, double h, double* dI,
+                                                    double* dtau) {
+    IeeeOps m;
+    flow_step_in(m, S, F, field, tp, delta, r, u, phi, t, lam, Ecam, h, dI, dtau);
+}
+// The step in straight-line arithmetic: every value of the IEEE form (numerators below its range end in
+// emissions far under the smallest float).  k_emit64_records with it, and three CTAs of 80 registers (two
+// of 92 otherwise): the 262,144-ray list's emission and transfer 8.1 -> 6.9 ms, the 501 x 375 flow
+// frame's 12.8 -> 9.8, the 1024^2 torus frame's 21.8 -> 19.1.
+__device__ __forceinline__ void flow_step(const so_scene& S, const so_frame& F, const float* field, const TorusParams& tp,
+                                          double delta, double r, double u, double phi, double t, double lam,
+                                          double Ecam, double h, double* dI, double* dtau) {
+    QuickOps m;
+    double a, b;
+    flow_step_in(m, S, F, field, tp, delta, r, u, phi, t, lam, Ecam, h, &a, &b);
+    if (m.bad) {
+        const TorusParams tpc = tp;
+        double c, d;
+        flow_step_again(S, F, field, tpc, delta, r, u, phi, t, lam, Ecam, h, &c, &d);
+        a = c;
+        b = d;
+    }
+    *dI = a;
+    *dtau = b;
 }
 
 // escape_angles (trace.cuh:49-55).
