@@ -110,7 +110,16 @@ struct HotScene {
     int max_steps, flow_on, disk_on;
 };
 
+// The hot flow's scene values in FP32 (rounded once, on the host) for flow_step32.
+struct Flow32 {
+    float a, r_flow_max, r_isco, rh, n0, n_index, theta0, theta_index, h_r, beta_p, kep, nu_obs, rg_cm;
+    float k2_l0, k2_dl;
+    int k2_n;
+    const float* k2_lntab;
+};
+
 struct TraceLaunch {
+    Flow32 flow32;
     HotScene hot;             // scene 0 and frame 0, for launches with hot_ok (one scene, one frame)
     int hot_ok;
     int disk_time;            // disk variant: the shading reads the coordinate time (disk turbulence)

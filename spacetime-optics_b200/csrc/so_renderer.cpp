@@ -396,6 +396,9 @@ void launch_common(so_renderer* r, TraceLaunch& L) {
              S.max_steps, S.flow_on, S.disk_on};
     L.hot_ok = 1;
     L.disk_time = S.disk_turb_amp > 0.f;
+    L.flow32 = {(float)S.a, (float)S.r_flow_max, (float)S.r_isco, (float)S.rh, (float)S.n0, (float)S.n_index,
+                (float)S.theta0, (float)S.theta_index, (float)S.h_r, (float)S.beta_p, (float)S.flow_kep,
+                (float)S.nu_obs, (float)S.rg_cm, S.k2_l0, S.k2_dl, S.k2_n, S.k2_lntab};
     const so_plasma& p = r->plasma;
     L.torus = p.model == SO_PLASMA_TORUS;
     L.n_modes = L.torus ? p.n_modes : 0;
