@@ -973,7 +973,7 @@ __global__ void __launch_bounds__(128) k_transfer64(const TraceLaunch L) {
     const bool skip = *(volatile unsigned long long*)&L.rec64_ctl[1] != 0ull;
     const unsigned long long cmask = (1ull << REC64_COUNT_BITS) - 1ull;
     unsigned long long n_att = 0, n_acc = 0, n_lim = 0, n_flow = 0;
-    const long long total = skip ? 0 : L.nrays;
+    const long long total = skip ? 0 : (L.nrays_dev ? (long long)*L.nrays_dev : L.nrays);
     for (long long jrel = (long long)blockIdx.x * blockDim.x + threadIdx.x; jrel < total;
          jrel += (long long)gridDim.x * blockDim.x) {
         const long long job = L.job0 + jrel;

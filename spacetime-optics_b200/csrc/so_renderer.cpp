@@ -53,6 +53,18 @@ double now_ms() {
 }
 }  // namespace
 
+// Device buffers of one chain of deferred FP64 passes (TraceLaunch's rec64 .. rec64_ctl).
+struct Records64 {
+    double* rec;
+    uint32_t* seg_next;
+    uint2* seg_meta;
+    Sample64* samp;
+    int* head;
+    long long seg_cap;
+    unsigned long long* ctl;
+    Counters* cnt;
+};
+
 struct so_renderer {
     int device = 0, num_sms = 148;
     cudaStream_t st = nullptr;
@@ -160,6 +172,13 @@ struct so_renderer {
     int waves64 = 0;                           // waves of the last deferred trace
     long long samples64 = 0;                   // samples of the last deferred trace (for the estimate)
     bool last_defer64 = false, last_emit64 = false;
+    // the band and re-trace rays of a mixed frame: their own record pool on the second stream
+    Records64 side{};
+    long long side_doubles = 0, side_jobs = 0;
+    double side_per_ray = 640.0;               // records per ray, doubled after a shortage
+    unsigned long long* h_side = nullptr;      // pinned: pool counters of the two launches (3 each)
+    cudaEvent_t ev_side = nullptr;
+    bool side_pending = false;
     long long list_rays = 0;                   // rays of the last so_trace_rays whose counters d_cnt holds
     std::vector<so_batch*> batches;            // live batches on this renderer (detached by so_destroy)
     std::string err;
@@ -243,6 +262,12 @@ void free_all(so_renderer* r) {
                    r->d_cnt64};
     for (void* p : p64)
         if (p) cudaFree(p);
+    void* ps64[] = {r->side.rec, r->side.seg_next, r->side.seg_meta, r->side.samp, r->side.head, r->side.ctl,
+                    r->side.cnt};
+    for (void* p : ps64)
+        if (p) cudaFree(p);
+    if (r->h_side) cudaFreeHost(r->h_side);
+    if (r->ev_side) cudaEventDestroy(r->ev_side);
     if (r->h_rec64) cudaFreeHost(r->h_rec64);
     if (r->ev_rec64) cudaEventDestroy(r->ev_rec64);
     for (cudaEvent_t e : r->ev64)
@@ -542,6 +567,12 @@ int ensure_records64(so_renderer* r, long long jobs, int per_job, int w, long lo
     return SO_OK;
 }
 
+// The renderer's record pool, as ensure_records64 set it up.
+Records64 main_records(const so_renderer* r) {
+    return {r->d_rec64, r->d_seg_next64, r->d_seg_meta64, r->d_samp64, r->d_job_head64, r->seg_cap64, r->d_rec64_ctl,
+            r->d_cnt64};
+}
+
 // Launches of the FP64 tracer.  A launch of at least kDeferMinJobs host-counted jobs on the
 // renderer's stream defers work out of the tracer when it is a torus-plasma launch with FP64 sums,
 // or a launch on the reference flow model: a recording pass (geometry only, one record per flow
@@ -556,9 +587,9 @@ int ensure_records64(so_renderer* r, long long jobs, int per_job, int w, long lo
 // ensure_records64 set up: per wave a recording pass, the sums (sums: 0 none, 1 FP64, 2 FP32), the
 // emission and ordered transfer (emit), and a replay pass that runs when the pool ran short (always,
 // without emit).  With `timed` the phases are bracketed by events (not inside a graph capture).
-// Each wave's pool counters go to h_rec64 for the shortage feedback and the statistics.
-int enqueue_deferred64(so_renderer* r, const TraceLaunch& L, int var, cudaStream_t s, long long wave, int w, int sums,
-                       bool emit, bool timed) {
+// Each wave's pool counters go to `ctl` (3 per wave).
+int enqueue_deferred64(so_renderer* r, const Records64& pool, const TraceLaunch& L, int var, cudaStream_t s,
+                       long long wave, int w, int sums, bool emit, bool timed, unsigned long long* ctl) {
     const int nw = (int)((L.nrays + wave - 1) / wave);
     if (nw > kMaxWaves64) return fail(r, SO_ERR_SIZE, "FP64 record pool: too many waves");
     if (timed) {
@@ -570,22 +601,22 @@ int enqueue_deferred64(so_renderer* r, const TraceLaunch& L, int var, cudaStream
     }
     for (int k = 0; k < nw; ++k) {
         const long long j0 = (long long)k * wave;
-        SO_CK(r, cudaMemsetAsync(r->d_rec64_ctl, 0, 3 * sizeof(unsigned long long), s));
-        SO_CK(r, cudaMemsetAsync(r->d_cnt64, 0, sizeof(Counters), s));
+        SO_CK(r, cudaMemsetAsync(pool.ctl, 0, 3 * sizeof(unsigned long long), s));
+        SO_CK(r, cudaMemsetAsync(pool.cnt, 0, sizeof(Counters), s));
         TraceLaunch L1 = L;
         L1.defer64 = 1;
         L1.emit32 = 0;
-        L1.counters = r->d_cnt64;
-        L1.rec64 = r->d_rec64;
+        L1.counters = pool.cnt;
+        L1.rec64 = pool.rec;
         L1.rec64_w = w;
         L1.job0 = j0;
         L1.nrays = std::min<long long>(wave, L.nrays - j0);
-        L1.seg_next64 = r->d_seg_next64;
-        L1.seg_meta64 = r->d_seg_meta64;
-        L1.samp64 = r->d_samp64;
-        L1.job_head64 = r->d_job_head64;
-        L1.seg_cap64 = r->seg_cap64;
-        L1.rec64_ctl = r->d_rec64_ctl;
+        L1.seg_next64 = pool.seg_next;
+        L1.seg_meta64 = pool.seg_meta;
+        L1.samp64 = pool.samp;
+        L1.job_head64 = pool.head;
+        L1.seg_cap64 = pool.seg_cap;
+        L1.rec64_ctl = pool.ctl;
         TraceLaunch L2 = L1;
         L2.defer64 = 2;
         L2.counters = L.counters;
@@ -615,10 +646,9 @@ int enqueue_deferred64(so_renderer* r, const TraceLaunch& L, int var, cudaStream
         e = launch_trace64(L2, var, r->num_sms, s);
         if (e != cudaSuccess) return cuda_fail(r, e, "tracer launch (replay pass)");
         if (ev) cudaEventRecord(ev[4], s);
-        SO_CK(r, cudaMemcpyAsync(r->h_rec64 + 3 * k, r->d_rec64_ctl, 3 * sizeof(unsigned long long),
+        SO_CK(r, cudaMemcpyAsync(ctl + 3 * k, pool.ctl, 3 * sizeof(unsigned long long),
                                  cudaMemcpyDeviceToHost, s));
     }
-    r->waves64 = nw;
     return SO_OK;
 }
 
@@ -636,7 +666,10 @@ int run_tracer(so_renderer* r, const TraceLaunch& L, cudaStream_t st = nullptr) 
         long long wave = 0;
         if (ensure_records64(r, L.nrays, per_job, w, &wave) == SO_OK) {
             r->samples64 = L.nrays * per_job;
-            if (int rc = enqueue_deferred64(r, L, var, s, wave, w, torus ? 1 : 0, emit_ok, true)) return rc;
+            if (int rc = enqueue_deferred64(r, main_records(r), L, var, s, wave, w, torus ? 1 : 0, emit_ok, true,
+                                            r->h_rec64))
+                return rc;
+            r->waves64 = (int)((L.nrays + wave - 1) / wave);
             SO_CK(r, cudaEventRecord(r->ev_rec64, s));
             r->rec64_pending = true;
             r->last_defer64 = true;
@@ -648,6 +681,70 @@ int run_tracer(so_renderer* r, const TraceLaunch& L, cudaStream_t st = nullptr) 
     cudaError_t e = launch_trace64(L, var, r->num_sms, s);
     if (e != cudaSuccess) return cuda_fail(r, e, "tracer launch");
     return SO_OK;
+}
+
+// Record pool of a mixed frame's band and re-trace lists (their counts are only on the device): room for
+// `rays` rays at side_per_ray records, within an eighth of the free device memory, and
+// chain heads for all of the frame's ns samples.  A list that runs short is traced again by the replay
+// pass (the same result, slower) and doubles the estimate for the next frames.
+int ensure_side(so_renderer* r, long long rays, long long ns) {
+    constexpr int w = REC64_W_FLOW;
+    Records64& p = r->side;
+    if (!r->h_side) {
+        SO_CK(r, cudaMallocHost((void**)&r->h_side, 6 * sizeof(unsigned long long)));
+        std::memset(r->h_side, 0, 6 * sizeof(unsigned long long));
+        SO_CK(r, cudaEventCreateWithFlags(&r->ev_side, cudaEventDisableTiming));
+    }
+    if (!p.ctl && dalloc(&p.ctl, 3) != cudaSuccess) return fail(r, SO_ERR_ALLOC, "side records: allocation");
+    if (!p.cnt && dalloc(&p.cnt, 1) != cudaSuccess) return fail(r, SO_ERR_ALLOC, "side records: allocation");
+    if (r->side_pending && cudaEventQuery(r->ev_side) == cudaSuccess) {
+        r->side_pending = false;
+        if (r->h_side[1] + r->h_side[4] > 0) r->side_per_ray *= 2.0;
+    }
+    cudaGetLastError();  // a pending event reports cudaErrorNotReady
+    const double seg_doubles = (double)REC_SEG * w;
+    long long want = (long long)((double)rays * (r->side_per_ray / REC_SEG + 1.0) * seg_doubles);
+    if (want > r->side_doubles) {
+        SO_CK(r, cudaStreamSynchronize(r->st));  // joined with the second stream at the end of each frame
+        void* ps[] = {p.rec, p.seg_next, p.seg_meta};
+        for (void* q : ps)
+            if (q) cudaFree(q);
+        p.rec = nullptr;
+        p.seg_next = nullptr;
+        p.seg_meta = nullptr;
+        r->side_doubles = 0;
+        size_t fr = 0, tot = 0;
+        SO_CK(r, cudaMemGetInfo(&fr, &tot));
+        want = std::min<long long>(want, (long long)(fr / 8 / (sizeof(double) + 1)));
+        const long long nseg = want / (REC_SEG * w);
+        if (nseg < 1 || dalloc(&p.rec, (size_t)want) != cudaSuccess || dalloc(&p.seg_next, (size_t)nseg) != cudaSuccess ||
+            dalloc(&p.seg_meta, (size_t)nseg) != cudaSuccess)
+            return fail(r, SO_ERR_ALLOC, "side records: device allocation");
+        r->side_doubles = want;
+    }
+    p.seg_cap = std::min<long long>(r->side_doubles / (REC_SEG * w), 0x7fffffffll);
+    if (ns > r->side_jobs) {
+        SO_CK(r, cudaStreamSynchronize(r->st));
+        if (p.head) cudaFree(p.head);
+        if (p.samp) cudaFree(p.samp);
+        p.head = nullptr;
+        p.samp = nullptr;
+        r->side_jobs = 0;
+        if (dalloc(&p.head, (size_t)ns) != cudaSuccess || dalloc(&p.samp, (size_t)ns) != cudaSuccess)
+            return fail(r, SO_ERR_ALLOC, "side records: chain heads");
+        r->side_jobs = ns;
+    }
+    return SO_OK;
+}
+
+// A list of the mixed frame (samples, counted on the device) through the FP64 tracer on the second stream:
+// by the deferred passes where `deferred`, else with the emission in the tracer.  `slot`: 0 the
+// band, 1 the re-trace.
+int run_side(so_renderer* r, const TraceLaunch& L, bool deferred, int slot) {
+    if (!deferred) return run_tracer(r, L, r->st2);
+    r->last_defer64 = false;
+    return enqueue_deferred64(r, r->side, L, VAR_RADIO, r->st2, L.nrays, REC64_W_FLOW, 0, true, false,
+                              r->h_side + 3 * slot);
 }
 
 // Escape (u, v) of the (W + 1) x (H + 1) pixel corners of the frame in d_frame (k_corners,
@@ -899,7 +996,21 @@ int trace_pass1_mixed(so_renderer* r, const so_frame& f, TraceLaunch& L) {
     // at 2048^2 210.3 / 207.4 / 210.3 ms, the vacuum shadow frame at 2048^2 one CTA 122.5 Mrays/s
     // against 119.8 with two; the images identical.
     Lb.ctas_per_sm = (L.torus && L.n_modes > 0) ? 2 : 1;
-    int rc = run_tracer(r, Lb, r->st2);
+    // On scenes without turbulence sums their emission is deferred too: a frame ends on the re-trace's longest
+    // ray (up to max_steps attempts), whose chain is shorter by the emission's, 16.0 -> 12.1 ms of
+    // the reference flow frame at 1024^2 (58.4 -> 54.2 ms).  Not with the sums: the deferred passes
+    // find no room on the SMs before the frame's own sums are done, and end as a tail (the 2048^2
+    // synchrotron frame 181 -> 185 ms).  Nor where the band (about 2 band_m times the critical
+    // curve's 33 M in area) is so much of the frame that its records would not fit.
+    bool side = variant_of(r->S) == VAR_RADIO && r->S.flow_on && !r->S.disk_on && !all64 && r->mixed.turbulence == 0 &&
+                !(L.torus && L.n_modes > 0) && r->S.max_steps < (1 << REC64_COUNT_BITS);
+    if (side) {
+        const double pix_m = f.pix * f.r;
+        const double rays = 2.0 * r->mixed.band_m * 33.0 / (pix_m * pix_m) * f.spp * 1.25 + (double)ns / 1000.0 + 2048.0;
+        side = rays < 0.25 * (double)ns + 4096.0 && ensure_side(r, (long long)std::min(rays, (double)ns), ns) == SO_OK;
+        if (!side) r->err.clear();
+    }
+    int rc = run_side(r, Lb, side, 0);
     if (rc) return rc;
     const bool torus_defer = variant_of(r->S) == VAR_RADIO && L.torus && L.n_modes > 0;
     const bool flow_defer = variant_of(r->S) == VAR_RADIO && !L.torus && r->S.flow_on && !all64;
@@ -944,8 +1055,12 @@ int trace_pass1_mixed(so_renderer* r, const so_frame& f, TraceLaunch& L) {
             Lr.list = r->d_redo;
             Lr.nrays_dev = &r->d_nlists[2];
             Lr.counters = &r->d_cnt3[1];
-            rc = run_tracer(r, Lr, r->st2);
+            rc = run_side(r, Lr, side, 1);
             if (rc) return rc;
+            if (side) {
+                SO_CK(r, cudaEventRecord(r->ev_side, r->st2));
+                r->side_pending = true;
+            }
             SO_CK(r, cudaEventRecord(r->ev_join, r->st2));
         }
         if (defer) {
@@ -1867,8 +1982,10 @@ int batch_enqueue(so_batch* b, float* d_px) {
     TraceLaunch L;
     batch_launch_desc(b, d_px, L);
     if (b->wave64 > 0) {
-        if (int rc = enqueue_deferred64(r, L, b->variant, r->st, b->wave64, b->w64, b->sums64, true, false))
+        if (int rc = enqueue_deferred64(r, main_records(r), L, b->variant, r->st, b->wave64, b->w64, b->sums64, true,
+                                        false, r->h_rec64))
             return rc;
+        r->waves64 = (int)((L.nrays + b->wave64 - 1) / b->wave64);
     } else {
         cudaError_t e = launch_trace64(L, b->variant, r->num_sms, r->st);
         if (e != cudaSuccess) return cuda_fail(r, e, "batch tracer launch");
