@@ -1,6 +1,6 @@
 // BF16 GEMM tile on the fifth-generation tensor cores: tcgen05.mma with both operands in shared
 // memory and the FP32 accumulator in tensor memory (TMEM), read back with tcgen05.ld for the
-// epilogue.  One CTA of 128 threads owns a 128 x BN output tile (BN <= 256 TMEM columns):
+// epilogue.  One CTA of 256 threads owns a 128 x BN output tile (BN <= 256 TMEM columns):
 //   * all threads stage A and B K-slices into shared memory (a ring of four, cp.async), in the K-major
 //     no-swizzle canonical layout: an 8-row x 16-byte "core matrix" is 128 contiguous bytes, the
 //     K-neighbouring core matrices of one 8-row group sit 128 B apart (leading byte offset) and the
@@ -8,7 +8,11 @@
 //   * thread 0 issues BK/16 tcgen05.mma (M=128, N=BN, K=16) per slice and commits them to the
 //     slice's mbarrier, so three slices load while the tensor core works on one;
 //   * after the last commit every warp reads its 32 TMEM lanes (= 32 output rows) with tcgen05.ld
-//     and applies the epilogue.
+//     and applies the epilogue; the two groups of four warps take alternate column blocks.
+//     The epilogue bounds the training products (a tanh and three stores per element against 64
+//     to 512 flops): twice the warps, 64-wide slices of the long reductions and the derivatives loaded
+//     ahead took a pass over 65,536 rays from 1.105 to 1.035 ms.  It stays latency-bound (DRAM 12 to
+//     17 %, issue 25 to 45 %); three CTAs of 128-wide tiles per SM were slower (1.09 ms).
 // Every mbarrier wait is bounded (about one second of %globaltimer); a wait that gives up writes
 // SO_ERR_WATCHDOG into *err, skips the epilogue and still frees the TMEM columns.
 #include "so_mlp.h"
@@ -19,11 +23,10 @@ namespace mlp {
 namespace {
 
 constexpr int BM = 128;
-constexpr int NT = 128;  // threads per CTA
-constexpr int NS = 4;    // K-slices in the shared-memory ring
+constexpr int NT = 256;  // threads per CTA: two groups of four warps (a group covers the tile's 128 rows)
+constexpr int NG = NT / 128;
 constexpr unsigned long long WAIT_NS = 1000000000ull;
-// shared tiles of the epilogue: bf16 [128][40] x 2 + bf16 [32][136] (or fp32 [128][36]), after the
-// [128][BN + 8] derivative tile of the backward epilogue
+// shared tiles of one group's epilogue: bf16 [128][40] x 2 + bf16 [32][136] (or fp32 [128][36])
 constexpr int EPI_SMEM = BM * 40 * 2 * 2 + 32 * 136 * 2;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -127,7 +130,8 @@ __device__ __forceinline__ void cp_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-template <int EPI>
+// NS: K-slices in the shared-memory ring.
+template <int EPI, int NS>
 __global__ void __launch_bounds__(NT) k_gemm_bf16(GemmArgs g, int BN, int BK, int tmem_cols) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ uint64_t bars[NS];
@@ -203,35 +207,33 @@ __global__ void __launch_bounds__(NT) k_gemm_bf16(GemmArgs g, int BN, int BK, in
         // (its TMEM lane), the values go to small shared tiles, and the block then stores whole
         // 16-byte row segments -- or, for the transposed outputs, whole column segments -- so every
         // global store instruction of a warp writes contiguous 128-byte lines.
-        const int r = warp * 32 + lane;
-        const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
-        uint8_t* ep = smem;
-        bf16* TD = nullptr;  // GELU_BWD: the tile's derivatives, [128][BN + 8]
-        if (EPI == EPI_GELU_BWD) {
-            TD = reinterpret_cast<bf16*>(ep);
-            const int segs = BN / 8;
-            for (int w = tid; w < BM * segs; w += NT) {
-                const int rr = w / segs, sg = w % segs;
-                const uint32_t dst = smem_u32(TD + rr * (BN + 8) + 8 * sg);
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst),
-                             "l"(g.d_in + (long)(m0 + rr) * g.ldd + n0 + 8 * sg)
-                             : "memory");
-            }
-            cp_commit();
-            ep += BM * (BN + 8) * 2;
-        }
+        const int group = warp >> 2, gtid = tid & 127;
+        const int r = (warp & 3) * 32 + lane;
+        const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+        uint8_t* ep = smem + group * EPI_SMEM;
         float* T32 = reinterpret_cast<float*>(ep);                // [128][36] fp32 (F32, SPLIT)
         bf16* T16 = reinterpret_cast<bf16*>(ep);                  // [128][40] bf16, row-major
         bf16* TG = T16 + BM * 40;                                 // [128][40] bf16, derivatives
         bf16* TT = TG + BM * 40;                                  // [32][136] bf16, transposed
-        if (EPI == EPI_GELU_BWD) {
-            cp_wait<0>();
-            __syncthreads();
-        }
+        // the group's own barrier (0 is __syncthreads)
+        auto group_sync = [&] {
+            if (group == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
+            else asm volatile("bar.sync 2, 128;" ::: "memory");
+        };
         const int cb = BN < 32 ? BN : 32;
-        for (int c = 0; c < BN; c += cb) {
+        uint4 dv[4];  // GELU_BWD: this row's derivatives of a column block (whole 32-byte sectors)
+        auto load_d = [&](int c) {
+            const uint4* src = reinterpret_cast<const uint4*>(g.d_in + (long)(m0 + r) * g.ldd + n0 + c);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (8 * i < cb) dv[i] = __ldg(src + i);
+        };
+        if (EPI == EPI_GELU_BWD && group * cb < BN) load_d(group * cb);
+        for (int c = group * cb; c < BN; c += cb * NG) {
             const int n = n0 + c;
-            for (int h = 0; h < cb; h += 16) {
+#pragma unroll
+            for (int h = 0; h < 32; h += 16) {
+                if (h >= cb) break;
                 float f[16];
                 tmem_ld16(lane_addr + c + h, f);
                 if (EPI == EPI_F32 || EPI == EPI_SPLIT) {
@@ -248,9 +250,8 @@ __global__ void __launch_bounds__(NT) k_gemm_bf16(GemmArgs g, int BN, int BK, in
                 } else {
                     __align__(16) bf16 o16[16], d16[16];
                     if (EPI == EPI_GELU_BWD) {
-                        const uint4* src = reinterpret_cast<const uint4*>(TD + r * (BN + 8) + c + h);
-                        *reinterpret_cast<uint4*>(d16) = src[0];
-                        *reinterpret_cast<uint4*>(d16 + 8) = src[1];
+                        *reinterpret_cast<uint4*>(d16) = dv[h / 8];
+                        *reinterpret_cast<uint4*>(d16 + 8) = dv[h / 8 + 1];
                     }
 #pragma unroll
                     for (int i = 0; i < 16; ++i) {
@@ -273,11 +274,12 @@ __global__ void __launch_bounds__(NT) k_gemm_bf16(GemmArgs g, int BN, int BK, in
                     }
                 }
             }
-            __syncthreads();
+            if (EPI == EPI_GELU_BWD && c + cb * NG < BN) load_d(c + cb * NG);  // the next block's, behind the stores
+            group_sync();
             if (EPI == EPI_F32 || EPI == EPI_SPLIT) {
                 float* base = g.out_f + (EPI == EPI_SPLIT ? blockIdx.z * g.split_stride : 0);
                 const int segs = cb / 4;
-                for (int w = tid; w < BM * segs; w += NT) {
+                for (int w = gtid; w < BM * segs; w += 128) {
                     const int rr = w / segs, sg = w % segs;
                     *reinterpret_cast<float4*>(base + (long)(m0 + rr) * g.ldf + n + 4 * sg) =
                         *reinterpret_cast<const float4*>(T32 + rr * 36 + 4 * sg);
@@ -285,7 +287,7 @@ __global__ void __launch_bounds__(NT) k_gemm_bf16(GemmArgs g, int BN, int BK, in
             }
             if (EPI == EPI_GELU || EPI == EPI_GELU_BWD) {
                 const int segs = cb / 8;
-                for (int w = tid; w < BM * segs; w += NT) {
+                for (int w = gtid; w < BM * segs; w += 128) {
                     const int rr = w / segs, sg = w % segs;
                     if (g.out_b)
                         *reinterpret_cast<uint4*>(g.out_b + (long)(m0 + rr) * g.ldob + n + 8 * sg) =
@@ -295,14 +297,14 @@ __global__ void __launch_bounds__(NT) k_gemm_bf16(GemmArgs g, int BN, int BK, in
                             *reinterpret_cast<const uint4*>(TG + rr * 40 + 8 * sg);
                 }
                 if (g.out_t) {
-                    for (int w = tid; w < cb * (BM / 8); w += NT) {
+                    for (int w = gtid; w < cb * (BM / 8); w += 128) {
                         const int j = w / (BM / 8), sg = w % (BM / 8);
                         *reinterpret_cast<uint4*>(g.out_t + (long)(n + j) * g.ldot + m0 + 8 * sg) =
                             *reinterpret_cast<const uint4*>(TT + j * 136 + 8 * sg);
                     }
                 }
             }
-            __syncthreads();
+            group_sync();
         }
     } else if (tid == 0 && g.err) {
         atomicExch(g.err, SO_ERR_WATCHDOG);
@@ -315,16 +317,16 @@ __global__ void __launch_bounds__(NT) k_gemm_bf16(GemmArgs g, int BN, int BK, in
     }
 }
 
-template <int EPI>
+template <int EPI, int NS = 4>
 int launch_epi(const GemmArgs& g, int BN, int BK, cudaStream_t st) {
     const int stage_bytes = NS * (BM + BN) * BK * 2;
-    const int epi_bytes = EPI_SMEM + (EPI == EPI_GELU_BWD ? BM * (BN + 8) * 2 : 0);
+    const int epi_bytes = NG * EPI_SMEM;
     const int smem = stage_bytes > epi_bytes ? stage_bytes : epi_bytes;
     const int cols = BN <= 32 ? 32 : BN <= 64 ? 64 : BN <= 128 ? 128 : 256;
-    if (cudaFuncSetAttribute(k_gemm_bf16<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+    if (cudaFuncSetAttribute(k_gemm_bf16<EPI, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
         return SO_ERR_CUDA;
     dim3 grid(g.M / BM, g.N / BN, g.splits);
-    k_gemm_bf16<EPI><<<grid, NT, smem, st>>>(g, BN, BK, cols);
+    k_gemm_bf16<EPI, NS><<<grid, NT, smem, st>>>(g, BN, BK, cols);
     return cudaGetLastError() == cudaSuccess ? SO_OK : SO_ERR_CUDA;
 }
 
@@ -378,6 +380,9 @@ int launch_gemm(const GemmArgs& g, cudaStream_t st, const char** why) {
             if (!g.out_f || g.ldf < g.N || g.ldf % 4 || !al16(g.out_f) ||
                 (g.splits > 1 && g.split_stride < (long)g.M * g.ldf) || g.split_stride % 4)
                 return bad("gemm: EPI_SPLIT needs out_f with 16-byte aligned rows and disjoint planes");
+            // long reductions: 64-wide slices (whole 128-byte lines of rows that lie far apart, half the
+            // barriers), three of them so that two CTAs of 96 KB still share an SM
+            if (kps % 64 == 0 && kps >= 512 && BN <= 128) return launch_epi<EPI_SPLIT, 3>(g, BN, 64, st);
             return launch_epi<EPI_SPLIT>(g, BN, BK, st);
         case EPI_SPLIT_T:
             if (!g.out_f || g.ldf < g.M || (g.splits > 1 && g.split_stride < (long)g.N * g.ldf))
