@@ -397,7 +397,7 @@ __device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
 
 // DEFER (deferred FP64 passes, radio only): 0 = emission in the tracer; 1 = recording pass on the torus
 // with its modes (geometry only: no emission code; records hold the advected azimuth), 4 = recording
-// pass of the flow form; 3 and 5 = the same two for a ray list (also record each step's crossings and
+// pass of the flow form (6: for few CTAs per SM); 3 and 5 = the same two for a ray list (also record each step's crossings and
 // write the rays' outputs without emission); 2 = replay pass.
 // HOT: one scene, whose values come from the launch descriptor (constant-bank operands) and not from the
 // ray's scene in memory; not for the radio kernels with the emission inside, where it made no difference.  TIME: the coordinate time is integrated (vacuum rays, and disks without turbulence,
@@ -405,12 +405,13 @@ __device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
 //
 // Register budget.  An SM's scheduler holds 3 warps at 168 registers, 4 at 128, so 128-thread CTAs come
 // three or four to an SM; which is better is what the extra warp hides against the spills it costs.
-// Measured (recording pass, three against four): the reference flow 501 x 375 frame 39.0 against 47.8 ms,
-// the 262,144-ray list 10.9 against 11.0, the 1024^2 torus frame 50.4 against 46.2 (the logarithm and
-// roots of the torus phase run on a third of the lanes, which the fourth warp hides); thin disk
-// 1280 x 720 x 2 19.9 against 21.9; 65,536 vacuum rays 2.8 against 3.1; five (96 registers) lose everywhere.
+// Measured, three against four: the 1024^2 torus frame's recording pass 50.4 against 46.2 ms, the 501 x 375
+// flow frame 74.9 against 73.3, the 262,144-ray flow list 17.7 against 17.3, thin disk 1280 x 720 x 2
+// 21.9 against 19.9; but a flow list held to few CTAs per SM (the mixed frame's band and re-trace, DEFER
+// 6: the chain's latency) 53.9 against 55.5 ms of the frame, and 65,536 vacuum rays 2.8 against 3.1.
+// Five (96 registers) lose everywhere.
 constexpr int tracer_ctas(int var, int defer) {
-    return defer == 1 || defer == 2 || defer == 3 || var == VAR_DISK ? 4 : 3;
+    return (defer >= 1 && defer <= 5) || var == VAR_DISK ? 4 : 3;
 }
 template <int VAR, bool EMIT32, int DEFER, bool HOT, bool TIME>
 __global__ void __launch_bounds__(128, tracer_ctas(VAR, DEFER)) k_trace64(const __grid_constant__ TraceLaunch L) {
@@ -450,7 +451,12 @@ __global__ void __launch_bounds__(128, tracer_ctas(VAR, DEFER)) k_trace64(const 
         __syncthreads();
     }
     const int lane = threadIdx.x & 31;
-    const long long total = L.nrays_dev ? (long long)*L.nrays_dev : L.nrays;
+    // A recording pass queues the samples of its jobs one by one (each has its own chain and end state):
+    // a lane that took whole jobs of an adaptive pass walked eight rays in a row, and 55 k such jobs do not
+    // even fill the lanes once.  Recording pass of the 501 x 375 flow frame's adaptive pass 39.0 -> 34.2 ms
+    // (the frame 82 -> 74.8), the flux frame of 160^2 pixels and two samples 17.1 -> 13.2 ms.
+    const int per = defer != 1 ? 1 : L.kind == RAYS_PIXELS ? L.spp : L.kind == RAYS_CHUNKS ? L.chunk : 1;
+    const long long total = (L.nrays_dev ? (long long)*L.nrays_dev : L.nrays) * per;
     // Short lists (re-trace lists, small ray lists) leave most lanes of the grid without a ray; then
     // only every stride-th lane takes rays, so the rays spread over more warps and each warp's
     // cooperative turbulence sums serve fewer lanes.  The same for every lane of the grid.
@@ -502,7 +508,8 @@ __global__ void __launch_bounds__(128, tracer_ctas(VAR, DEFER)) k_trace64(const 
         const bool need = !active && !exhausted && worker;
         const bool grab = need && chunk_left == 0;
         const unsigned m = __ballot_sync(FULL, grab);
-        unsigned long long j = (unsigned long long)(job - L.job0) + 1;  // the next job of the lane's grab
+        // the next job of the lane's grab
+        unsigned long long j = (unsigned long long)(job - L.job0) * per + (defer == 1 ? sample : 0) + 1;
         if (m) {
             const int leader = __ffs(m) - 1;
             unsigned long long base = 0;
@@ -519,9 +526,13 @@ __global__ void __launch_bounds__(128, tracer_ctas(VAR, DEFER)) k_trace64(const 
                 if (j >= (unsigned long long)total) {
                     exhausted = true;
                 } else {
-                    job = L.job0 + (long long)j;
                     active = true;
                     sample = 0;
+                    if (defer == 1 && per > 1) {
+                        sample = (int)(j % per);
+                        j /= per;
+                    }
+                    job = L.job0 + (long long)j;
                     const JobPlace q = job_place(L, job);
                     fidx = q.fidx;
                     pix = q.pix;
@@ -532,7 +543,7 @@ __global__ void __launch_bounds__(128, tracer_ctas(VAR, DEFER)) k_trace64(const 
                         x = L.x[job];
                         yv = L.y[job];
                     } else {
-                        pixel_point(L, L.frames[fidx], pix, sbase, &x, &yv);
+                        pixel_point(L, L.frames[fidx], pix, sbase + sample, &x, &yv);
                     }
                     S = &L.scenes[L.frame_scene[fidx]];
                     F = &L.frames[fidx];
@@ -643,8 +654,7 @@ __global__ void __launch_bounds__(128, tracer_ctas(VAR, DEFER)) k_trace64(const 
             continue;
         // sample finished
         if (defer == 1) {
-            // recording pass: the sample's chain is closed with its end state, and the job's next
-            // sample, if any, opens its own
+            // recording pass: the sample's chain is closed with its end state
             const long long sid = (job - L.job0) * jobs_n + sample;
             L.job_head64[sid] = rinline ? -2 : rhead;
             if (rinline) atomicAdd(&L.rec64_ctl[1], 1ull);
@@ -662,13 +672,6 @@ __global__ void __launch_bounds__(128, tracer_ctas(VAR, DEFER)) k_trace64(const 
             // a ray list's outputs of the ray without emission; the transfer writes its intensity and,
             // where the opacity cut ends it earlier, what the tracer reports for it there
             if (list_rec) list_out(L.out, job, fate, R.ncross, th, ph, R.nacc, R.natt, cr, cg);
-            if ((L.kind == RAYS_PIXELS || L.kind == RAYS_CHUNKS) && ++sample < jobs_n) {
-                double x, yv;
-                pixel_point(L, *F, pix, sbase + sample, &x, &yv);
-                ray_init<VAR>(R, *S, *F, x, yv);
-                chain_start(sample);
-                continue;
-            }
             active = false;
             continue;
         }
@@ -1179,6 +1182,8 @@ cudaError_t launch_trace64(const TraceLaunch& L, int variant, int num_sms, cudaS
             if (L.defer64 == 1 && torus)
                 return L.hot_ok ? go(k_trace64<VAR_RADIO, false, 1, true, true>)
                                 : go(k_trace64<VAR_RADIO, false, 1, false, true>);
+            if (L.defer64 == 1 && L.hot_ok && L.ctas_per_sm > 0 && L.ctas_per_sm < 4)
+                return go(k_trace64<VAR_RADIO, false, 6, true, true>);
             if (L.defer64 == 1)
                 return L.hot_ok ? go(k_trace64<VAR_RADIO, false, 4, true, true>)
                                 : go(k_trace64<VAR_RADIO, false, 4, false, true>);
