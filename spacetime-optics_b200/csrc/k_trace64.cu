@@ -747,16 +747,19 @@ __global__ void __launch_bounds__(128, tracer_ctas(VAR, DEFER)) k_trace64(const 
 // modes, so an FMA of the phase reads three different registers and the pipe starves on the
 // register file: 0.77 T mode-positions/s whatever the number of positions and warps.  Here a thread
 // owns kTurb64P positions and all threads read the same mode, a broadcast of 16-byte shared loads
-// whose values the positions reuse.  The 1024^2 synchrotron frame's sums: 181.8 -> 155.0 ms (0.95 T
-// mode-positions/s, 2.5 cycles per FP64 instruction against 2.2 of independent FMAs); with 4
-// positions 176 (unrolled twice 165), with 6 166, with 10 in CTAs of 128 172.
+// whose values the positions reuse, the next mode's loaded meanwhile.  What is left is decided by how the
+// operands fall on the register banks, and many registers leave the choice: eleven positions in one CTA
+// of 384 threads (154 registers).  The 1024^2 synchrotron frame's sums: warp form 181.8 ms; 11 positions
+// 142.8 (1.03 T mode-positions/s, 2.26 cycles per FP64 instruction against 2.18 of independent FMAs),
+// 12 143.3, 16 (236 registers, 256 threads) 146.0, 8 (two CTAs of 256, unrolled twice) 144.6; without
+// the load ahead 8 155, 12 150; under 100 registers 165 to 176 whatever the shape.
 //
 // The order of warp_sums is kept: partial sum l takes modes l, l + 32, l + 64, ..., and the butterfly
 // (xor 16, 8, 4, 2, 1) adds the partials as a balanced tree whose leaves are l in bit-reversed order.
 // Visiting l in that order, a binary counter of five pending subtrees per position adds the same
 // pairs.  Slots past a chain's last record (the segment's count) are summed at the origin and left
 // unwritten.
-constexpr int kTurb64P = 8;
+constexpr int kTurb64P = 11;
 // acc[j] += w cos_turns(k . X_j + p), written stage by stage over the positions (the operations of
 // cos_turns, so_kerr.cuh), so that the P chains interleave.
 template <int P>
@@ -790,9 +793,9 @@ __device__ __forceinline__ void add_mode(double kx, double ky, double kz, double
     EACH acc[j] = fma(w, bitsd(dbits(c[j]) ^ ((dbits(s[j]) & 1ull) << 63)), acc[j]);
 #undef EACH
 }
-constexpr int kTurb64Threads = 256;
+constexpr int kTurb64Threads = 384;
 constexpr int kModeStride = 6;  // doubles per mode in shared memory: k, phase, amplitude, pad
-__global__ void __launch_bounds__(kTurb64Threads) k_turb64_records(const TraceLaunch L) {
+__global__ void __launch_bounds__(kTurb64Threads, 1) k_turb64_records(const TraceLaunch L) {
     extern __shared__ __align__(16) double smem64[];
     const int n = L.n_modes;
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
@@ -827,12 +830,26 @@ __global__ void __launch_bounds__(kTurb64Threads) k_turb64_records(const TraceLa
         for (unsigned b = 0; b < 32; ++b) {
 #pragma unroll
             for (int j = 0; j < P; ++j) acc[j] = 0.0;
-#pragma unroll 1
-            for (int i = (int)(__brev(b) >> 27); i < n; i += 32) {
+            int i = (int)(__brev(b) >> 27);
+            double2 k01, k23;
+            double w = 0.0;
+            k01 = k23 = make_double2(0.0, 0.0);
+            if (i < n) {
                 const double2* q = reinterpret_cast<const double2*>(smem64 + kModeStride * i);
-                const double2 k01 = q[0], k23 = q[1];
-                const double w = smem64[kModeStride * i + 4];
+                k01 = q[0];
+                k23 = q[1];
+                w = smem64[kModeStride * i + 4];
+            }
+#pragma unroll 1
+            for (; i < n; i += 32) {
+                const int nx = i + 32 < n ? i + 32 : i;
+                const double2* q = reinterpret_cast<const double2*>(smem64 + kModeStride * nx);
+                const double2 n01 = q[0], n23 = q[1];
+                const double nw = smem64[kModeStride * nx + 4];
                 add_mode<P>(k01.x, k01.y, k23.x, k23.y, w, px, py, pz, acc);
+                k01 = n01;
+                k23 = n23;
+                w = nw;
             }
 #pragma unroll
             for (int lev = 0; lev < 5; ++lev) {
