@@ -6,10 +6,12 @@
 //              half of a layer, read the accumulators from tensor memory (tcgen05.ld), add the bias,
 //              tanh-form GELU in half precision, round to BF16 and write the next layer's input in
 //              place; after the head, write the 16 FP32 outputs to global memory.
-//   warp 16    (one elected thread): streams the packed BF16 weights through a ring of six 16 KB
+//   warp 16    (one elected thread): issues the tensor-core MMAs (tcgen05.mma, M=128, K=16, N=128 or
+//              16 for the head), each weight chunk serving both 128-ray halves of the tile;
+//   warp 17    (one elected thread): streams the packed BF16 weights through a ring of six 16 KB
 //              shared-memory buffers with bulk copies (cp.async.bulk, mbarrier transaction counts,
-//              no multicast) and issues the tensor-core MMAs (tcgen05.mma, M=128, K=16, N=128 or
-//              16 for the head), each weight chunk serving both 128-ray halves of the tile.
+//              no multicast).  With one thread for both, the refill's wait for the previous chunk's
+//              MMAs left the tensor core a chunk deep at most: a megaray 0.905 ms, 0.745 apart.
 //
 // Each layer is cut into output halves n0, n1 (128 columns, TMEM columns [0,128) and [128,256) of
 // each ray half) and input halves k0, k1, and its four blocks run in the order (n0,k0), (n1,k0),
@@ -35,7 +37,8 @@ namespace {
 
 constexpr int TILE = 256;      // rays per tile (two MMA halves of 128)
 constexpr int NEPI = 512;      // epilogue threads (16 warps)
-constexpr int NTHR = NEPI + 32;
+constexpr int NTHR = NEPI + 32;       // 2-SM form: one control warp
+constexpr int NTHR1 = NEPI + 64;      // 1-SM form: an MMA warp and a weight-stream warp
 #ifndef SO_FUSED_NBUF
 #define SO_FUSED_NBUF 6
 #define SO_FUSED_CHUNK_K 64
@@ -204,7 +207,7 @@ __device__ __forceinline__ void epilogue32(const uint32_t (&v)[32], const __half
 }
 
 
-__global__ void __launch_bounds__(NTHR, 1) k_mlp_fused(const FusedArgs a) {
+__global__ void __launch_bounds__(NTHR1, 1) k_mlp_fused(const FusedArgs a) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ uint64_t full[NBUF], empty[NBUF], acc_ready[2], epi_done[2];
     __shared__ uint32_t tmem_slot;
@@ -234,7 +237,7 @@ __global__ void __launch_bounds__(NTHR, 1) k_mlp_fused(const FusedArgs a) {
         abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    for (int i = tid; i < NHID * HID / 2; i += NTHR) {
+    for (int i = tid; i < NHID * HID / 2; i += NTHR1) {
         const int l = i / (HID / 2), c = i % (HID / 2);
         const float* b = a.params + a.bias_off[l] + 2 * c;
         bias2[l][c] = __floats2half2_rn(b[0], b[1]);
@@ -244,18 +247,31 @@ __global__ void __launch_bounds__(NTHR, 1) k_mlp_fused(const FusedArgs a) {
     fence_after();
     const uint32_t tmem = tmem_slot;
 
-    if (warp == NEPI / 32) {
-        // ---- weight stream and MMA issue (one thread) ----
+    if (warp == NEPI / 32 + 1) {
+        // ---- weight stream (one thread): chunk q goes into buffer q % NBUF once the MMAs of chunk
+        // q - NBUF are done
         if (lane == 0) {
             const long long total = (long long)my_tiles * a.nchunks;
-            long long issued = 0, consumed = 0;
-            auto load = [&](long long q) {
+            long long q = 0;
+            for (; q < total; ++q) {
                 const int b = (int)(q % NBUF);
+                if (q >= NBUF && !bar_wait(&empty[b], (uint32_t)(((q - NBUF) / NBUF) & 1), &abort_flag)) break;
                 const FusedChunk& c = a.chunks[q % a.nchunks];
                 bar_expect_tx(&full[b], (uint32_t)c.bytes);
                 bulk_g2s(wbuf + b * CHUNK_BYTES, a.wpack + c.offset, (uint32_t)c.bytes, &full[b]);
-            };
-            for (; issued < total && issued < NBUF - 1; ++issued) load(issued);
+            }
+            // copies still in flight land before the CTA exits
+            for (long long p = q > NBUF ? q - NBUF : 0; p < q; ++p) {
+                volatile int never = 0;
+                bar_wait(&full[p % NBUF], (uint32_t)((p / NBUF) & 1), &never);
+            }
+            if (q < total && a.err) atomicExch(a.err, SO_ERR_WATCHDOG);
+        }
+    } else if (warp == NEPI / 32) {
+        // ---- MMA issue (one thread; a thread that also refilled the ring would wait for each chunk's MMAs
+        // before it could queue the next) ----
+        if (lane == 0) {
+            long long consumed = 0;
             uint32_t ph_epi[2] = {0, 0};
             bool ok = true;
             // Descriptors are linear in the address (the start field holds address >> 4), so each
@@ -285,16 +301,6 @@ __global__ void __launch_bounds__(NTHR, 1) k_mlp_fused(const FusedArgs a) {
                     }
                     mma_commit(&empty[b]);
                     ++consumed;
-                    // refill: chunk `issued` goes into the buffer of chunk issued - NBUF, the one
-                    // issued just before chunk q (the tensor core still has q queued meanwhile)
-                    if (issued < total) {
-                        const long long prev = issued - NBUF;
-                        if (prev >= 0 &&
-                            !bar_wait(&empty[issued % NBUF], (uint32_t)((prev / NBUF) & 1), &abort_flag))
-                            return false;
-                        load(issued);
-                        ++issued;
-                    }
                 }
                 return true;
             };
@@ -316,11 +322,6 @@ __global__ void __launch_bounds__(NTHR, 1) k_mlp_fused(const FusedArgs a) {
                     if (ok && !head) ok = block(1, 1, K, idesc);
                     if (ok && !head) mma_commit(&acc_ready[1]);
                 }
-            }
-            // copies still in flight land before the CTA exits
-            for (long long q = consumed; q < issued; ++q) {
-                volatile int never = 0;
-                bar_wait(&full[q % NBUF], (uint32_t)((q / NBUF) & 1), &never);
             }
             if (!ok && a.err) atomicExch(a.err, SO_ERR_WATCHDOG);
         }
@@ -838,7 +839,7 @@ int launch_mlp_fused(const FusedArgs& a, int num_sms, cudaStream_t st) {
         return SO_ERR_CUDA;
     const long long ntiles = (a.n + TILE - 1) / TILE;
     const int grid = (int)(ntiles < num_sms ? ntiles : num_sms);
-    k_mlp_fused<<<grid, NTHR, SMEM_BYTES, st>>>(a);
+    k_mlp_fused<<<grid, NTHR1, SMEM_BYTES, st>>>(a);
     return cudaGetLastError() == cudaSuccess ? SO_OK : SO_ERR_CUDA;
 }
 
