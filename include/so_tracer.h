@@ -238,7 +238,7 @@ typedef struct so_mixed_opts {
     double tol_approach;     /* tolerance of the FP64 approach (0 = 10 x the scene's render.tolerance: the
                               * far field carries no emission, and the synchrotron frame's image moves
                               * by 2e-5 L1 and keeps every class for it, at 7 % less frame time) */
-    int t32_blocks;          /* FP32 tracer: resident 128-thread CTAs per SM, 4, 5 or 6 (0 = 4) */
+    int t32_blocks;          /* FP32 tracer: resident 128-thread CTAs per SM, 4, 5 or 6 (0 = 5) */
     int turbulence;          /* torus turbulence of the FP32 rays: 0 = deferred (the tracer records its
                               * emitting flow steps, one batched kernel sums the Fourier modes at all of
                               * them, one kernel runs the ordered transfer per ray; the record pool takes

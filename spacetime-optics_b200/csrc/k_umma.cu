@@ -110,18 +110,18 @@ __device__ __forceinline__ void tmem_ld16(uint32_t addr, float* f) {
 }
 
 // Stage rows [0, rows) x K-slice [k0, k0 + BK) of a K-major global matrix into the canonical
-// layout with asynchronous 16-byte copies (cp.async, L2 only).  One item moves 32 bytes (two
-// core-matrix rows along K); a warp's 32 items cover 8 rows x 4 K-pairs, so the shared-memory
-// side touches every bank once per 128 bytes.
+// layout with asynchronous 16-byte copies (cp.async, L2 only).  Neighbouring lanes copy neighbouring
+// 16-byte pieces of a row, so that a warp's copy reads whole sectors (with lanes on 32-byte steps every
+// sector was requested twice); on the shared-memory side eight rows x the slice's pieces are
+// contiguous.
 __device__ __forceinline__ void stage_async(uint8_t* sm, const bf16* g, long ld, int rows, int k0, int BK, int tid) {
-    const int nkq = BK >> 4;
-    const int items = rows * nkq;
+    const int sh = BK == 16 ? 1 : BK == 32 ? 2 : 3;  // log2 of the 16-byte pieces in a row of the slice
+    const int items = rows << sh;
     for (int w = tid; w < items; w += NT) {
-        const int rr = w & 7, kq = (w >> 3) % nkq, rg = (w >> 3) / nkq;
-        const bf16* src = g + (long)(rg * 8 + rr) * ld + k0 + kq * 16;
-        const uint32_t dst = smem_u32(sm + rg * (BK * 16) + kq * 256 + rr * 16);
+        const int kp = w & ((1 << sh) - 1), row = w >> sh;
+        const bf16* src = g + (long)row * ld + k0 + kp * 8;
+        const uint32_t dst = smem_u32(sm + (row >> 3) * (BK * 16) + kp * 128 + (row & 7) * 16);
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 128), "l"(src + 8) : "memory");
     }
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }

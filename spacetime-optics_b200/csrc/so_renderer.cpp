@@ -934,7 +934,9 @@ int trace_pass1_mixed(so_renderer* r, const so_frame& f, TraceLaunch& L) {
         std::memcpy(r->approach_key, key, sizeof key);
     }
     L.approach_it = r->approach_it;
-    L.t32_min_blocks = r->mixed.t32_blocks > 0 ? r->mixed.t32_blocks : 4;
+    // five CTAs of 96 registers per SM: reference flow frame 1024^2 50.9 ms (four 54.1, six 50.7), 2048^2
+    // synchrotron frame 180.3 (181.3, 182.8)
+    L.t32_min_blocks = r->mixed.t32_blocks > 0 ? r->mixed.t32_blocks : 5;
     L.t32_max_att = r->mixed.fp32_max_attempts > 0 ? r->mixed.fp32_max_attempts : 2000;
     // outgoing rays beyond every emitter cannot come back: the FP32 tracer ends them as escaped
     double r_emit = 0.0;
