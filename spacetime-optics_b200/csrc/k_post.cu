@@ -186,23 +186,43 @@ __global__ void __launch_bounds__(256) k_lum_hist(const float* __restrict__ lum,
         if (sh[b]) atomicAdd(&hist[b], sh[b]);
 }
 
-// The bin holding rank k (one thread: at most 4096 bins), then the rank inside it.  After pass 0
-// the rank is min(n - 1, (size_t)(percentile (n - 1))) of the n significant values, as the host's.
-__global__ void k_lum_pick(const unsigned* __restrict__ hist, int pass, double percentile, LumStat* st) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    const int nb = pass == 0 ? 4096 : pass == 1 ? 2048 : 256;
-    unsigned long long k = st->k;
-    if (pass == 0) {
-        unsigned long long n = 0;
-        for (int b = 0; b < nb; ++b) n += hist[b];
-        st->nsig = n;
-        if (n == 0) return;
-        k = (unsigned long long)(percentile * (double)(n - 1));
-        if (k > n - 1) k = n - 1;
+// The bin holding rank k, then the rank inside it.  After pass 0 the rank is
+// min(n - 1, (size_t)(percentile (n - 1))) of the n significant values, as the host's.  One block: each
+// thread adds its share of the (at most 4096) bins, a scan finds the share holding the rank, and that
+// thread walks it.  One thread walking all of it took 0.24 to 0.30 ms a frame, bound by the latency of its
+// dependent loads (the 1280 x 720 thin disk's frame 18.7 -> 18.4 ms).
+__global__ void __launch_bounds__(256) k_lum_pick(const unsigned* __restrict__ hist, int pass, double percentile,
+                                                  LumStat* st) {
+    __shared__ unsigned long long wsum[8];
+    const int per = pass == 0 ? 16 : pass == 1 ? 8 : 1, nb = 256 * per;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    unsigned long long own = 0;
+    for (int i = 0; i < per; ++i) own += hist[t * per + i];
+    unsigned long long incl = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
     }
-    if (st->nsig == 0) return;
-    unsigned long long cum = 0;
-    int b = 0;
+    if (lane == 31) wsum[warp] = incl;
+    unsigned long long k = st->k, nsig = st->nsig;
+    __syncthreads();
+    unsigned long long total = 0, cum = incl - own;
+    for (int w = 0; w < 8; ++w) {
+        if (w < warp) cum += wsum[w];
+        total += wsum[w];
+    }
+    if (pass == 0) {
+        nsig = total;
+        if (t == 0) st->nsig = nsig;
+        if (nsig == 0) return;
+        k = (unsigned long long)(percentile * (double)(nsig - 1));
+        if (k > nsig - 1) k = nsig - 1;
+    }
+    if (nsig == 0) return;
+    const bool last = t == 255 && k >= total;
+    if (!last && (k < cum || k >= cum + own)) return;
+    int b = t * per;
     for (; b < nb - 1; ++b) {
         if (cum + hist[b] > k) break;
         cum += hist[b];
@@ -223,7 +243,7 @@ cudaError_t post_luminance(const float4* img, long long n, int radio, float hide
         cudaError_t e = cudaMemsetAsync(s.hist, 0, LUM_HIST * sizeof(unsigned), st);
         if (e != cudaSuccess) return e;
         k_lum_hist<<<LUM_BLOCKS, 256, 0, st>>>(s.lum, n, s.stat, pass, s.hist);
-        k_lum_pick<<<1, 32, 0, st>>>(s.hist, pass, percentile, s.stat);
+        k_lum_pick<<<1, 256, 0, st>>>(s.hist, pass, percentile, s.stat);
     }
     return cudaGetLastError();
 }
