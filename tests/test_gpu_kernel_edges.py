@@ -73,3 +73,42 @@ def test_disk_with_and_without_time(so, orc, turb):
         assert np.array_equal(k[key], o[key]), key
     I0, I1 = o["I"].astype(np.float64), k["I"].astype(np.float64)
     assert I0.max() > 0 and np.abs(I0 - I1).max() <= 1e-5 * I0.max()
+
+
+@pytest.mark.parametrize("spp", [2, 3, 4, 32])
+def test_transfer_samples_per_job(so, spp):
+    """The ordered transfer takes a lane per sample at 2, 4, .. 32 samples a job and one thread otherwise: the
+    frame with a record pool (4320 jobs: enough to defer) equals the one whose pool is too small (the replay
+    pass) bit for bit."""
+    imgs = []
+    for pool in ({}, {"pool_mb": 0.001}):
+        sh = so.Shot("m87_reference_flow.ini", ["camera.width=72", "camera.height=60", f"render.spp={spp}",
+                                                f"render.spp_max={spp}"])
+        r = so.Renderer(sh.scene, sh.tables, sh.settings)
+        r.set_precision(so.abi.SO_PREC_FP64, **pool)
+        img, _, st = r.render(sh.frame(0))
+        r.close()
+        assert (st.rec64_short > 0) == bool(pool)
+        imgs.append(img)
+    assert imgs[0][..., 0].max() > 0 and np.array_equal(*imgs)
+
+
+@pytest.mark.parametrize("band_m", [0.05, 0.6])
+def test_mixed_flow_band_deferred(so, band_m):
+    """A mixed reference-flow frame's band rays, their emission deferred to passes of their own, equal bit for
+    bit the same rays of a frame whose band covers the field (emission in the tracer)."""
+    n = 128
+    sh = so.Shot("m87_reference_flow.ini", [f"camera.width={n}", f"camera.height={n}", "render.spp=1",
+                                            "render.spp_max=1"])
+    r = so.Renderer(sh.scene, sh.tables, sh.settings)
+    f = sh.frame(0)
+    r.set_precision(so.abi.SO_PREC_MIXED, band_m=band_m)
+    a, _, _ = r.render(f)
+    fa, band = r.last_fates(n * n)
+    r.set_precision(so.abi.SO_PREC_MIXED, band_m=1e6)
+    b, _, _ = r.render(f)
+    fb, every = r.last_fates(n * n)
+    r.close()
+    assert every.all() and 0 < band.sum() < n * n // 4
+    a, b = a.reshape(n * n, -1), b.reshape(n * n, -1)
+    assert b[band, 0].max() > 0 and np.array_equal(a[band], b[band]) and np.array_equal(fa[band], fb[band])
