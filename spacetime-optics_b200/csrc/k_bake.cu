@@ -14,7 +14,7 @@
 // run's eight corners into gradient vectors in shared memory, which all the texels of the run read
 // back.  About 24 of 128 cells are hashed per 32 texels and generation.  What depends on the row
 // alone (radius, retarded time, shear, generation) is computed once per row, and the sine and cosine
-// of phi come from a table turned by the row's shear angle.  113 M texels: 11.3 -> 6.4 ms on the B200
+// of phi come from a table turned by the row's shear angle.  113 M texels: 11.3 -> 6.2 ms on the B200
 // (integer pipe 72 % -> 46 %, FMA pipe 39 %, issue 77 %).
 //
 // The float operations of a texel are those of the reference's noise in their order (its gradient is
