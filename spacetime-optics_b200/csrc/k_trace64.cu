@@ -408,10 +408,11 @@ __device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
 // Measured, three against four: the 1024^2 torus frame's recording pass 50.4 against 46.2 ms, the 501 x 375
 // flow frame 74.9 against 73.3, the 262,144-ray flow list 17.7 against 17.3, thin disk 1280 x 720 x 2
 // 21.9 against 19.9; but a flow list held to few CTAs per SM (the mixed frame's band and re-trace, DEFER
-// 6: the chain's latency) 53.9 against 55.5 ms of the frame, and 65,536 vacuum rays 2.8 against 3.1.
+// 6: the chain's latency) 53.9 against 55.5 ms of the frame, 65,536 vacuum rays 2.8 against 3.1, and
+// thin-disk frames that three CTAs per SM hold (also DEFER 6) 1.60 against 1.86 ms.
 // Five (96 registers) lose everywhere.
 constexpr int tracer_ctas(int var, int defer) {
-    return (defer >= 1 && defer <= 5) || var == VAR_DISK ? 4 : 3;
+    return (defer >= 1 && defer <= 5) || (var == VAR_DISK && defer != 6) ? 4 : 3;
 }
 template <int VAR, bool EMIT32, int DEFER, bool HOT, bool TIME>
 __global__ void __launch_bounds__(128, tracer_ctas(VAR, DEFER)) k_trace64(const __grid_constant__ TraceLaunch L) {
@@ -1213,6 +1214,12 @@ cudaError_t launch_trace64(const TraceLaunch& L, int variant, int num_sms, cudaS
             return L.hot_ok ? go(k_trace64<VAR_VACUUM, false, 0, true, false>)
                             : go(k_trace64<VAR_VACUUM, false, 0, false, false>);
         case VAR_DISK:
+            // Jobs that three CTAs per SM hold at once end with their longest ray, whose chain is shorter at
+            // 168 registers (51,200 pixels of two samples 1.60 ms against 1.86 with four CTAs); with
+            // more jobs than that four CTAs win (76,800 pixels 2.06 against 2.25 ms).
+            if (L.nrays <= (long long)num_sms * 3 * tpb)
+                return L.disk_time || !L.hot_ok ? go(k_trace64<VAR_DISK, false, 6, false, true>)
+                                                : go(k_trace64<VAR_DISK, false, 6, true, false>);
             if (L.disk_time || !L.hot_ok) return go(k_trace64<VAR_DISK, false, 0, false, true>);
             return go(k_trace64<VAR_DISK, false, 0, true, false>);
         default:

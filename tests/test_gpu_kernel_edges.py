@@ -112,3 +112,22 @@ def test_mixed_flow_band_deferred(so, band_m):
     assert every.all() and 0 < band.sum() < n * n // 4
     a, b = a.reshape(n * n, -1), b.reshape(n * n, -1)
     assert b[band, 0].max() > 0 and np.array_equal(a[band], b[band]) and np.array_equal(fa[band], fb[band])
+
+
+@pytest.mark.parametrize("ini,over", [("thin_disk_4096.ini", "disk.turbulence=0"), ("thin_disk_4096.ini", "disk.turbulence=0.6"),
+                                      ("m87_reference_flow.ini", "camera.incl=163"),
+                                      ("synchrotron_1024.ini", "so.modes=8")])
+def test_launch_shape_changes_no_ray(so, ini, over):
+    """A list that three CTAs per SM hold at once runs with 168 registers, a longer one with 128: every output
+    of 60,000 rays in one call equals that of the same rays in calls of 20,000 bit for bit."""
+    sh = so.Shot(ini, ["camera.width=250", "camera.height=240", over])
+    r = so.Renderer(sh.scene, sh.tables, sh.settings)
+    r.set_plasma(sh.plasma())
+    r.set_flow_noise(so.abi.SO_FLOW_NOISE_INLINE)
+    f = sh.frame(0)
+    X, Y = so.pixel_centres(f, 250, 240)
+    a = r.trace_rays(f, X, Y)
+    parts = [r.trace_rays(f, X[i:i + 20000], Y[i:i + 20000]) for i in range(0, 60000, 20000)]
+    r.close()
+    for key in ("fate", "ncross", "theta", "phi", "I", "n_accepted", "n_attempts"):
+        assert np.array_equal(a[key], np.concatenate([p[key] for p in parts]), equal_nan=True), key
