@@ -397,8 +397,9 @@ __device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
 
 // DEFER (deferred FP64 passes, radio only): 0 = emission in the tracer; 1 = recording pass on the torus
 // with its modes (geometry only: no emission code; records hold the advected azimuth), 4 = recording
-// pass of the flow form (6: for few CTAs per SM); 3 and 5 = the same two for a ray list (also record each step's crossings and
-// write the rays' outputs without emission); 2 = replay pass.
+// pass of the flow form; 3 and 5 = the same two for a ray list (also record each step's crossings and
+// write the rays' outputs without emission); 8, 6, 9 and 7 = these four (and 6 the disk) for launches of few
+// rays, at 168 registers; 2 = replay pass.
 // HOT: one scene, whose values come from the launch descriptor (constant-bank operands) and not from the
 // ray's scene in memory; not for the radio kernels with the emission inside, where it made no difference.  TIME: the coordinate time is integrated (vacuum rays, and disks without turbulence,
 // never read it).
@@ -407,9 +408,11 @@ __device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
 // three or four to an SM; which is better is what the extra warp hides against the spills it costs.
 // Measured, three against four: the 1024^2 torus frame's recording pass 50.4 against 46.2 ms, the 501 x 375
 // flow frame 74.9 against 73.3, the 262,144-ray flow list 17.7 against 17.3, thin disk 1280 x 720 x 2
-// 21.9 against 19.9; but a flow list held to few CTAs per SM (the mixed frame's band and re-trace, DEFER
-// 6: the chain's latency) 53.9 against 55.5 ms of the frame, 65,536 vacuum rays 2.8 against 3.1, and
-// thin-disk frames that three CTAs per SM hold (also DEFER 6) 1.60 against 1.86 ms.
+// 21.9 against 19.9; but a flow list held to few CTAs per SM (the mixed frame's band and re-trace: the
+// chain's latency) 53.9 against 55.5 ms of the frame, 65,536 vacuum rays 2.8 against 3.1, and launches
+// whose rays three CTAs per SM hold at once, which end with their longest ray (DEFER 6 to 9): the 160 x 160 x
+// 2 light curve 11.9 against 12.5 ms, flow lists of 5,000 and 56,000 rays 3.1 and 5.1 against 3.6 and 5.7
+// (60,000, just above, at four 5.8), a 94 x 66 x 2 torus frame 4.1 against 4.6, 256 x 200 x 2 disk 1.60 against 1.86.
 // Five (96 registers) lose everywhere.
 constexpr int tracer_ctas(int var, int defer) {
     return (defer >= 1 && defer <= 5) || (var == VAR_DISK && defer != 6) ? 4 : 3;
@@ -419,9 +422,9 @@ __global__ void __launch_bounds__(128, tracer_ctas(VAR, DEFER)) k_trace64(const 
     extern __shared__ double smem[];
     constexpr int defer = (VAR == VAR_RADIO && !EMIT32) ? (DEFER >= 3 ? 1 : DEFER) : 0;
     constexpr bool emit = defer != 1;
-    constexpr bool list_rec = defer == 1 && (DEFER == 3 || DEFER == 5);  // the recording pass of a ray list
+    constexpr bool list_rec = defer == 1 && (DEFER == 3 || DEFER == 5 || DEFER == 7 || DEFER == 9);  // the recording pass of a ray list
     constexpr bool hot = HOT && (VAR != VAR_RADIO || defer == 1);
-    constexpr bool torus_rec = defer == 1 && (DEFER == 1 || DEFER == 3);
+    constexpr bool torus_rec = defer == 1 && (DEFER == 1 || DEFER == 3 || DEFER >= 8);
     // the replay pass behind the deferred emission runs only when the recording pass left samples
     // without records (the same value for every thread: the whole grid returns)
     if (defer == 2 && L.replay_if_short && *(volatile unsigned long long*)&L.rec64_ctl[1] == 0ull) return;
@@ -1209,6 +1212,8 @@ cudaError_t launch_trace64(const TraceLaunch& L, int variant, int num_sms, cudaS
         kern<<<(int)grid, tpb, smem, st>>>(L);
         return cudaGetLastError();
     };
+    // samples (the recording passes queue them singly) that three CTAs per SM hold at once: see tracer_ctas
+    const bool few = L.nrays * job_samples(L) <= (long long)num_sms * 3 * tpb;
     switch (variant) {
         case VAR_VACUUM:
             return L.hot_ok ? go(k_trace64<VAR_VACUUM, false, 0, true, false>)
@@ -1224,14 +1229,19 @@ cudaError_t launch_trace64(const TraceLaunch& L, int variant, int num_sms, cudaS
             return go(k_trace64<VAR_DISK, false, 0, true, false>);
         default:
             if (emit32) return go(k_trace64<VAR_RADIO, true, 0, false, true>);
+            if (L.defer64 == 1 && L.hot_ok && (few || (!torus && L.ctas_per_sm > 0 && L.ctas_per_sm < 4))) {
+                if (L.kind == RAYS_LIST)
+                    return torus ? go(k_trace64<VAR_RADIO, false, 9, true, true>)
+                                 : go(k_trace64<VAR_RADIO, false, 7, true, true>);
+                return torus ? go(k_trace64<VAR_RADIO, false, 8, true, true>)
+                             : go(k_trace64<VAR_RADIO, false, 6, true, true>);
+            }
             if (L.defer64 == 1 && L.kind == RAYS_LIST)  // always one scene's (run_tracer)
                 return torus ? go(k_trace64<VAR_RADIO, false, 3, true, true>)
                              : go(k_trace64<VAR_RADIO, false, 5, true, true>);
             if (L.defer64 == 1 && torus)
                 return L.hot_ok ? go(k_trace64<VAR_RADIO, false, 1, true, true>)
                                 : go(k_trace64<VAR_RADIO, false, 1, false, true>);
-            if (L.defer64 == 1 && L.hot_ok && L.ctas_per_sm > 0 && L.ctas_per_sm < 4)
-                return go(k_trace64<VAR_RADIO, false, 6, true, true>);
             if (L.defer64 == 1)
                 return L.hot_ok ? go(k_trace64<VAR_RADIO, false, 4, true, true>)
                                 : go(k_trace64<VAR_RADIO, false, 4, false, true>);
