@@ -194,7 +194,10 @@ int fail(so_renderer* r, int code, const std::string& msg) {
     else g_init_error = msg;
     return code;
 }
+// (An error that was reported or has a fall-back is taken off the runtime too: it would be read again, as
+// the status of the next kernel launch.)
 int cuda_fail(so_renderer* r, cudaError_t e, const char* what) {
+    cudaGetLastError();
     return fail(r, SO_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 #define SO_CK(r, x)                                      \
@@ -205,7 +208,9 @@ int cuda_fail(so_renderer* r, cudaError_t e, const char* what) {
 
 template <typename T>
 cudaError_t dalloc(T** p, size_t n) {
-    return cudaMalloc((void**)p, std::max<size_t>(n, 1) * sizeof(T));
+    const cudaError_t e = cudaMalloc((void**)p, std::max<size_t>(n, 1) * sizeof(T));
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
 }
 
 int variant_of(const so_scene& S) {
@@ -496,8 +501,8 @@ int ensure_records64(so_renderer* r, long long jobs, int per_job, int w, long lo
     if (!r->h_rec64) {
         SO_CK(r, cudaMallocHost((void**)&r->h_rec64, 3 * kMaxWaves64 * sizeof(unsigned long long)));
         std::memset(r->h_rec64, 0, 3 * kMaxWaves64 * sizeof(unsigned long long));
-        SO_CK(r, cudaEventCreateWithFlags(&r->ev_rec64, cudaEventDisableTiming));
     }
+    if (!r->ev_rec64) SO_CK(r, cudaEventCreateWithFlags(&r->ev_rec64, cudaEventDisableTiming));
     if (!r->d_rec64_ctl && dalloc(&r->d_rec64_ctl, 3) != cudaSuccess)
         return fail(r, SO_ERR_ALLOC, "FP64 record pool: allocation");
     if (!r->d_cnt64 && dalloc(&r->d_cnt64, 1) != cudaSuccess) return fail(r, SO_ERR_ALLOC, "FP64 record pool: allocation");
@@ -693,8 +698,8 @@ int ensure_side(so_renderer* r, long long rays, long long ns) {
     if (!r->h_side) {
         SO_CK(r, cudaMallocHost((void**)&r->h_side, 6 * sizeof(unsigned long long)));
         std::memset(r->h_side, 0, 6 * sizeof(unsigned long long));
-        SO_CK(r, cudaEventCreateWithFlags(&r->ev_side, cudaEventDisableTiming));
     }
+    if (!r->ev_side) SO_CK(r, cudaEventCreateWithFlags(&r->ev_side, cudaEventDisableTiming));
     if (!p.ctl && dalloc(&p.ctl, 3) != cudaSuccess) return fail(r, SO_ERR_ALLOC, "side records: allocation");
     if (!p.cnt && dalloc(&p.cnt, 1) != cudaSuccess) return fail(r, SO_ERR_ALLOC, "side records: allocation");
     if (r->side_pending && cudaEventQuery(r->ev_side) == cudaSuccess) {
@@ -825,8 +830,8 @@ int ensure_records(so_renderer* r, long long ns) {
     if (!r->h_seg) {
         SO_CK(r, cudaMallocHost((void**)&r->h_seg, 2 * sizeof(unsigned long long)));
         r->h_seg[0] = r->h_seg[1] = 0;
-        SO_CK(r, cudaEventCreateWithFlags(&r->ev_seg, cudaEventDisableTiming));
     }
+    if (!r->ev_seg) SO_CK(r, cudaEventCreateWithFlags(&r->ev_seg, cudaEventDisableTiming));
     if (r->seg_pending && cudaEventQuery(r->ev_seg) == cudaSuccess) {
         r->seg_pending = false;
         if (r->h_seg[1] > 0) r->rec_per_ray *= 2.0;
@@ -905,13 +910,12 @@ int trace_pass1_mixed(so_renderer* r, const so_frame& f, TraceLaunch& L) {
             return fail(r, SO_ERR_ALLOC, "mixed path: device allocation");
         r->mixed_cap = ns;
     }
-    if (!r->d_nlists) {
-        if (dalloc(&r->d_nlists, NLISTS) != cudaSuccess || (!r->d_band && dalloc(&r->d_band, BAND_N) != cudaSuccess))
-            return fail(r, SO_ERR_ALLOC, "mixed path: device allocation");
-        if (int rc = ensure_side_queue(r)) return rc;
-        SO_CK(r, cudaEventCreate(&r->ev32[0]));
-        SO_CK(r, cudaEventCreate(&r->ev32[1]));
-    }
+    if ((!r->d_nlists && dalloc(&r->d_nlists, NLISTS) != cudaSuccess) ||
+        (!r->d_band && dalloc(&r->d_band, BAND_N) != cudaSuccess))
+        return fail(r, SO_ERR_ALLOC, "mixed path: device allocation");
+    if (int rc = ensure_side_queue(r)) return rc;
+    for (cudaEvent_t& e : r->ev32)
+        if (!e) SO_CK(r, cudaEventCreate(&e));
     if (r->band_a != r->S.a || r->band_th != f.th) {
         std::vector<float> tab = band_table(r->S.a, f.th);
         SO_CK(r, cudaMemcpyAsync(r->d_band, tab.data(), BAND_N * sizeof(float), cudaMemcpyHostToDevice, r->st));
@@ -1655,7 +1659,7 @@ int so_trace_rays(so_renderer* r, const so_frame* f, int n, const double* x, con
         r->d_rays = nullptr;
         r->ray_cap = 0;
         if (dalloc(&r->d_x, n) != cudaSuccess || dalloc(&r->d_y, n) != cudaSuccess ||
-            cudaMalloc(&r->d_rays, ray_bytes(n)) != cudaSuccess)
+            dalloc((char**)&r->d_rays, ray_bytes(n)) != cudaSuccess)
             return fail(r, SO_ERR_ALLOC, "so_trace_rays: device allocation");
         r->ray_cap = n;
     }

@@ -51,7 +51,9 @@ struct Rng {
 
 template <class T>
 cudaError_t dalloc(T** p, size_t n) {
-    return cudaMalloc((void**)p, n * sizeof(T));
+    const cudaError_t e = cudaMalloc((void**)p, n * sizeof(T));
+    if (e != cudaSuccess) cudaGetLastError();  // reported here: not to the next launch
+    return e;
 }
 
 }  // namespace
@@ -799,7 +801,7 @@ int so_sur_gemm(const void* d_a, const void* d_b, const float* d_bias, float* d_
     g.ldf = layout == 2 ? M : N;
     g.split_stride = (long)M * N;
     int* d_err = nullptr;
-    if (cudaMalloc(&d_err, sizeof(int)) != cudaSuccess) return SO_ERR_ALLOC;
+    if (dalloc(&d_err, 1) != cudaSuccess) return SO_ERR_ALLOC;
     cudaMemset(d_err, 0, sizeof(int));
     g.err = d_err;
     const char* why = nullptr;

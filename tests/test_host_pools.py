@@ -1,0 +1,76 @@
+"""Record pools of the deferred passes: what the host code does when memory is short, limited or has run out.
+The library runs in a child process on a CUDA runtime without a device (fake_cudart.cpp): kernels do
+nothing, so only allocations, launches and statuses mean anything."""
+import json
+import os
+import shutil
+import subprocess
+import sys
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+PRELUDE = """
+import ctypes as C, json, sys
+import numpy as np
+sys.path.insert(0, %r)
+import conftest
+so = conftest.load_package()
+rt = C.CDLL(sys.argv[1])
+for name in ("fake_mallocs", "fake_graphs", "fake_launches"):
+    getattr(rt, name).restype = C.c_longlong
+for name in ("fake_held", "fake_largest"):
+    getattr(rt, name).restype = C.c_size_t
+rt.fake_memory.argtypes = [C.c_size_t]
+rt.fake_fail_in.argtypes = [C.c_longlong]
+rt.fake_counts.argtypes = [C.c_int] + [C.c_ulonglong] * 3
+MIXED, FP64 = so.abi.SO_PREC_MIXED, so.abi.SO_PREC_FP64
+def flow(n):
+    sh = so.Shot("m87_reference_flow.ini", ["camera.width=%%d" %% n, "camera.height=%%d" %% n, "render.spp=1",
+                                            "render.spp_max=1"])
+    return so.Renderer(sh.scene, sh.tables, sh.settings), sh.frame(0)
+def frame(r, f):
+    # status of one frame into a buffer of the renderer's size, and what it allocated and launched
+    px = np.zeros(r.settings.W * r.settings.H * 4, np.float32)
+    m, l = rt.fake_mallocs(), rt.fake_launches()
+    rc = so.lib().so_render_device(r.h, C.byref(f), px.ctypes.data_as(C.c_void_p), None)
+    return rc, rt.fake_mallocs() - m, rt.fake_launches() - l
+"""
+
+
+@pytest.fixture(scope="module")
+def host(tmp_path_factory):
+    if shutil.which("g++") is None:
+        pytest.skip("needs g++")
+    lib = str(tmp_path_factory.mktemp("rt") / "fake_cudart.so")
+    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-o", lib, os.path.join(HERE, "fake_cudart.cpp")],
+                   check=True)
+
+    def run(body):
+        p = subprocess.run([sys.executable, "-c", PRELUDE % HERE + body, lib], env=dict(os.environ, LD_PRELOAD=lib),
+                           capture_output=True, text=True, timeout=300)
+        assert p.returncode == 0, p.stderr[-3000:]
+        return json.loads(p.stdout)
+    return run
+
+
+@pytest.mark.parametrize("prec,spare", [("MIXED", 8), ("FP64", 8)])
+def test_failed_allocation_leaves_no_error(host, prec, spare):
+    """Whichever allocation of a first reference flow frame fails, the frame is rendered (those of the FP64
+    passes' pools, `spare` of them: the rays then run in the tracer) or refused, and the next one is rendered."""
+    out, codes = host("""
+out = []
+for k in range(40):
+    r, f = flow(64)
+    r.set_precision(%s)
+    rt.fake_fail_in(k)
+    first = frame(r, f)[0]
+    rt.fake_fail_in(-1)
+    out.append((first, frame(r, f)[0]))
+    r.close()
+print(json.dumps([out, [0, so.abi.SO_ERR_ALLOC, so.abi.SO_ERR_CUDA]]))
+""" % prec)
+    n = max([i + 1 for i, (a, b) in enumerate(out) if a] + [0])
+    assert all(a in codes and b == 0 for a, b in out)
+    assert sum(a == 0 for a, _ in out[:max(n, spare)]) >= spare
