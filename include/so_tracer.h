@@ -260,7 +260,11 @@ typedef struct so_mixed_opts {
                               * FP32 rays that each fit (the image does not depend on the split).  Also
                               * caps the plain FP64 tracer's record pool (torus plasma, in either
                               * precision), beyond which samples are summed in the tracer: the same
-                              * sums, bit for bit, at lower occupancy */
+                              * sums, bit for bit, at lower occupancy; and the pool of a mixed frame's
+                              * band and re-traced rays without turbulence sums (otherwise an eighth
+                              * of the free device memory at most), where a list that does not fit
+                              * is traced again, the same rays bit for bit.  Each pool has the limit
+                              * to itself; their lists of one entry per sample come on top */
     int fp32_max_attempts;   /* FP32 attempts after which a ray is handed to the FP64 re-trace (0 = 2000:
                               * the FP32 controller stalls on a few rays far from the critical curve,
                               * which the FP64 tracer finishes normally; at 2048^2 the synchrotron

@@ -174,7 +174,7 @@ struct so_renderer {
     bool last_defer64 = false, last_emit64 = false;
     // the band and re-trace rays of a mixed frame: their own record pool on the second stream
     Records64 side{};
-    long long side_doubles = 0, side_jobs = 0;
+    long long side_jobs = 0;                   // chain heads
     double side_per_ray = 640.0;               // records per ray, doubled after a shortage
     unsigned long long* h_side = nullptr;      // pinned: pool counters of the two launches (3 each)
     cudaEvent_t ev_side = nullptr;
@@ -689,9 +689,9 @@ int run_tracer(so_renderer* r, const TraceLaunch& L, cudaStream_t st = nullptr) 
 }
 
 // Record pool of a mixed frame's band and re-trace lists (their counts are only on the device): room for
-// `rays` rays at side_per_ray records, within an eighth of the free device memory, and
-// chain heads for all of the frame's ns samples.  A list that runs short is traced again by the replay
-// pass (the same result, slower) and doubles the estimate for the next frames.
+// `rays` rays at side_per_ray records, within an eighth of the free device memory and
+// so_mixed_opts.pool_mb, and chain heads for all of the frame's ns samples.  A list that runs short is traced
+// again by the replay pass (the same result, slower) and doubles the estimate for the next frames.
 int ensure_side(so_renderer* r, long long rays, long long ns) {
     constexpr int w = REC64_W_FLOW;
     Records64& p = r->side;
@@ -707,9 +707,12 @@ int ensure_side(so_renderer* r, long long rays, long long ns) {
         if (r->h_side[1] + r->h_side[4] > 0) r->side_per_ray *= 2.0;
     }
     cudaGetLastError();  // a pending event reports cudaErrorNotReady
-    const double seg_doubles = (double)REC_SEG * w;
-    long long want = (long long)((double)rays * (r->side_per_ray / REC_SEG + 1.0) * seg_doubles);
-    if (want > r->side_doubles) {
+    const double per_seg = REC_SEG * w * sizeof(double) + sizeof(uint32_t) + sizeof(uint2);
+    long long limit = 0x7fffffffll;
+    if (r->mixed.pool_mb > 0.0)
+        limit = std::min<long long>(limit, std::max<long long>(1, (long long)(r->mixed.pool_mb * 1048576.0 / per_seg)));
+    const long long want = std::min<long long>(limit, (long long)((double)rays * (r->side_per_ray / REC_SEG + 1.0)));
+    if (want > p.seg_cap || limit < p.seg_cap) {
         SO_CK(r, cudaStreamSynchronize(r->st));  // joined with the second stream at the end of each frame
         void* ps[] = {p.rec, p.seg_next, p.seg_meta};
         for (void* q : ps)
@@ -717,17 +720,15 @@ int ensure_side(so_renderer* r, long long rays, long long ns) {
         p.rec = nullptr;
         p.seg_next = nullptr;
         p.seg_meta = nullptr;
-        r->side_doubles = 0;
+        p.seg_cap = 0;
         size_t fr = 0, tot = 0;
         SO_CK(r, cudaMemGetInfo(&fr, &tot));
-        want = std::min<long long>(want, (long long)(fr / 8 / (sizeof(double) + 1)));
-        const long long nseg = want / (REC_SEG * w);
-        if (nseg < 1 || dalloc(&p.rec, (size_t)want) != cudaSuccess || dalloc(&p.seg_next, (size_t)nseg) != cudaSuccess ||
-            dalloc(&p.seg_meta, (size_t)nseg) != cudaSuccess)
+        const long long nseg = std::min<long long>(want, (long long)(0.125 * (double)fr / per_seg));
+        if (nseg < 1 || dalloc(&p.rec, (size_t)nseg * REC_SEG * w) != cudaSuccess ||
+            dalloc(&p.seg_next, (size_t)nseg) != cudaSuccess || dalloc(&p.seg_meta, (size_t)nseg) != cudaSuccess)
             return fail(r, SO_ERR_ALLOC, "side records: device allocation");
-        r->side_doubles = want;
+        p.seg_cap = nseg;
     }
-    p.seg_cap = std::min<long long>(r->side_doubles / (REC_SEG * w), 0x7fffffffll);
     if (ns > r->side_jobs) {
         SO_CK(r, cudaStreamSynchronize(r->st));
         if (p.head) cudaFree(p.head);

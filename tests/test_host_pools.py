@@ -74,3 +74,22 @@ print(json.dumps([out, [0, so.abi.SO_ERR_ALLOC, so.abi.SO_ERR_CUDA]]))
     n = max([i + 1 for i, (a, b) in enumerate(out) if a] + [0])
     assert all(a in codes and b == 0 for a, b in out)
     assert sum(a == 0 for a, _ in out[:max(n, spare)]) >= spare
+
+
+def test_pool_limit_holds_for_every_pool(host):
+    """so_mixed_opts.pool_mb = 2 on a mixed reference-flow frame: no block above 2 MiB (the frame's own are
+    smaller), neither on a new renderer nor on one that rendered without a limit before."""
+    fresh, free, lowered = host("""
+r, f = flow(64)
+r.set_precision(MIXED, pool_mb=2.0)
+out = [(frame(r, f)[0], rt.fake_largest())]
+r.close()
+r, f = flow(64)
+r.set_precision(MIXED)
+out.append((frame(r, f)[0], rt.fake_largest()))
+r.set_precision(MIXED, pool_mb=2.0)
+out.append((frame(r, f)[0], rt.fake_largest()))
+print(json.dumps(out))
+""")
+    assert fresh[0] == free[0] == lowered[0] == 0
+    assert fresh[1] <= 2 << 20 and lowered[1] <= 2 << 20 < free[1]
