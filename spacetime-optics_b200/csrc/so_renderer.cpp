@@ -174,7 +174,7 @@ struct so_renderer {
     bool last_defer64 = false, last_emit64 = false;
     // the band and re-trace rays of a mixed frame: their own record pool on the second stream
     Records64 side{};
-    long long side_jobs = 0;                   // chain heads
+    long long side_target = 0, side_jobs = 0;  // segments asked for (free memory may have given fewer), chain heads
     double side_per_ray = 640.0;               // records per ray, doubled after a shortage
     unsigned long long* h_side = nullptr;      // pinned: pool counters of the two launches (3 each)
     cudaEvent_t ev_side = nullptr;
@@ -712,7 +712,10 @@ int ensure_side(so_renderer* r, long long rays, long long ns) {
     if (r->mixed.pool_mb > 0.0)
         limit = std::min<long long>(limit, std::max<long long>(1, (long long)(r->mixed.pool_mb * 1048576.0 / per_seg)));
     const long long want = std::min<long long>(limit, (long long)((double)rays * (r->side_per_ray / REC_SEG + 1.0)));
-    if (want > p.seg_cap || limit < p.seg_cap) {
+    // grow to a larger estimate, by a quarter more (frames of a zoom differ little); shrink only to a lowered
+    // limit; where free memory was the bound, the same estimate finds the pool as large as it gets
+    if (want > r->side_target || limit < p.seg_cap) {
+        const long long ask = std::min<long long>(limit, want + want / 4);
         SO_CK(r, cudaStreamSynchronize(r->st));  // joined with the second stream at the end of each frame
         void* ps[] = {p.rec, p.seg_next, p.seg_meta};
         for (void* q : ps)
@@ -721,13 +724,15 @@ int ensure_side(so_renderer* r, long long rays, long long ns) {
         p.seg_next = nullptr;
         p.seg_meta = nullptr;
         p.seg_cap = 0;
+        r->side_target = 0;
         size_t fr = 0, tot = 0;
         SO_CK(r, cudaMemGetInfo(&fr, &tot));
-        const long long nseg = std::min<long long>(want, (long long)(0.125 * (double)fr / per_seg));
+        const long long nseg = std::min<long long>(ask, (long long)(0.125 * (double)fr / per_seg));
         if (nseg < 1 || dalloc(&p.rec, (size_t)nseg * REC_SEG * w) != cudaSuccess ||
             dalloc(&p.seg_next, (size_t)nseg) != cudaSuccess || dalloc(&p.seg_meta, (size_t)nseg) != cudaSuccess)
             return fail(r, SO_ERR_ALLOC, "side records: device allocation");
         p.seg_cap = nseg;
+        r->side_target = ask;
     }
     if (ns > r->side_jobs) {
         SO_CK(r, cudaStreamSynchronize(r->st));

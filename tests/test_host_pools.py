@@ -93,3 +93,26 @@ print(json.dumps(out))
 """)
     assert fresh[0] == free[0] == lowered[0] == 0
     assert fresh[1] <= 2 << 20 and lowered[1] <= 2 << 20 < free[1]
+
+
+def test_side_pool_is_kept_from_frame_to_frame(host):
+    """Later frames of a renderer allocate nothing: where free memory (300 MB) bounds the side passes' pool, and,
+    but for one or two steps of growth, where each of 24 frames zooms in by 1 %."""
+    capped, zoomed = host("""
+rt.fake_memory(rt.fake_held() + (300 << 20))
+r, f = flow(64)
+r.set_precision(MIXED)
+capped = [frame(r, f)[:2] for i in range(5)]
+r.close()
+rt.fake_memory(64 << 30)
+r, f = flow(512)
+r.set_precision(MIXED)
+zoomed = []
+for i in range(24):
+    zoomed.append(frame(r, f)[:2])
+    f.pix *= 0.99
+print(json.dumps([capped, zoomed]))
+""")
+    assert all(rc == 0 for rc, _ in capped + zoomed)
+    assert capped[0][1] > 0 and sum(m for _, m in capped[1:]) == 0
+    assert sum(m > 0 for _, m in zoomed[1:]) <= 2
