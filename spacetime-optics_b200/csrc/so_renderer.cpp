@@ -176,6 +176,8 @@ struct so_renderer {
     Records64 side{};
     long long side_target = 0, side_jobs = 0;  // segments asked for (free memory may have given fewer), chain heads
     double side_per_ray = 640.0;               // records per ray, doubled after a shortage
+    long long side_rays = 0, side_max_rays = 0x7fffffffffffffffll;  // rays of the last frame with a pool; the most that get one
+    bool side_bounded = false;                 // the last such frame's pool was smaller than its need
     unsigned long long* h_side = nullptr;      // pinned: pool counters of the two launches (3 each)
     cudaEvent_t ev_side = nullptr;
     bool side_pending = false;
@@ -691,7 +693,9 @@ int run_tracer(so_renderer* r, const TraceLaunch& L, cudaStream_t st = nullptr) 
 // Record pool of a mixed frame's band and re-trace lists (their counts are only on the device): room for
 // `rays` rays at side_per_ray records, within an eighth of the free device memory and
 // so_mixed_opts.pool_mb, and chain heads for all of the frame's ns samples.  A list that runs short is traced
-// again by the replay pass (the same result, slower) and doubles the estimate for the next frames.
+// again by the replay pass (the same result, slower).  Its frame doubles the estimate for the next ones where
+// the pool was all that had been asked for; where memory or the limit had bounded it, frames of as many rays
+// get no pool from then on: their lists run in the tracer, which costs less than recording them in vain.
 int ensure_side(so_renderer* r, long long rays, long long ns) {
     constexpr int w = REC64_W_FLOW;
     Records64& p = r->side;
@@ -704,14 +708,19 @@ int ensure_side(so_renderer* r, long long rays, long long ns) {
     if (!p.cnt && dalloc(&p.cnt, 1) != cudaSuccess) return fail(r, SO_ERR_ALLOC, "side records: allocation");
     if (r->side_pending && cudaEventQuery(r->ev_side) == cudaSuccess) {
         r->side_pending = false;
-        if (r->h_side[1] + r->h_side[4] > 0) r->side_per_ray *= 2.0;
+        if (r->h_side[1] + r->h_side[4] > 0) {
+            if (r->side_bounded) r->side_max_rays = std::min(r->side_max_rays, r->side_rays - 1);
+            else r->side_per_ray *= 2.0;
+        }
     }
     cudaGetLastError();  // a pending event reports cudaErrorNotReady
+    if (rays > r->side_max_rays) return SO_ERR_SIZE;
     const double per_seg = REC_SEG * w * sizeof(double) + sizeof(uint32_t) + sizeof(uint2);
     long long limit = 0x7fffffffll;
     if (r->mixed.pool_mb > 0.0)
         limit = std::min<long long>(limit, std::max<long long>(1, (long long)(r->mixed.pool_mb * 1048576.0 / per_seg)));
-    const long long want = std::min<long long>(limit, (long long)((double)rays * (r->side_per_ray / REC_SEG + 1.0)));
+    const double need = (double)rays * (r->side_per_ray / REC_SEG + 1.0);
+    const long long want = (long long)std::min((double)limit, need);
     // grow to a larger estimate, by a quarter more (frames of a zoom differ little); shrink only to a lowered
     // limit; where free memory was the bound, the same estimate finds the pool as large as it gets
     if (want > r->side_target || limit < p.seg_cap) {
@@ -745,6 +754,8 @@ int ensure_side(so_renderer* r, long long rays, long long ns) {
             return fail(r, SO_ERR_ALLOC, "side records: chain heads");
         r->side_jobs = ns;
     }
+    r->side_rays = rays;
+    r->side_bounded = (double)p.seg_cap < need;
     return SO_OK;
 }
 
@@ -1735,7 +1746,10 @@ int so_set_precision(so_renderer* r, int precision, const so_mixed_opts* opts) {
         return fail(r, SO_ERR_ARG, "so_mixed_opts.pool_mb: 0 .. 1e7");
     if (opts && opts->records_per_ray > 0.0) r->rec_per_ray = opts->records_per_ray;
     r->precision = precision;
-    if (opts) r->mixed = *opts;
+    if (opts) {
+        r->mixed = *opts;
+        r->side_max_rays = 0x7fffffffffffffffll;  // another limit, band or depth
+    }
     return SO_OK;
 }
 

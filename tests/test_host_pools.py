@@ -116,3 +116,34 @@ print(json.dumps([capped, zoomed]))
     assert all(rc == 0 for rc, _ in capped + zoomed)
     assert capped[0][1] > 0 and sum(m for _, m in capped[1:]) == 0
     assert sum(m > 0 for _, m in zoomed[1:]) <= 2
+
+
+def test_side_pool_that_cannot_grow(host):
+    """Every list of every frame runs short.  A pool that may grow doubles; one bounded by free memory (300 MB) or by
+    pool_mb neither grows nor records in vain: from the second frame on the rays run in the tracer (six
+    launches fewer a frame, three a list), until so_set_precision gives another limit."""
+    grown, free, limited, again = host("""
+rt.fake_counts(1, 1, 1, 1)
+r, f = flow(64)
+r.set_precision(MIXED)
+grown = []
+for i in range(3):
+    frame(r, f)
+    grown.append(rt.fake_largest())
+r.close()
+def run(pool_mb):
+    r, f = flow(64)
+    r.set_precision(MIXED, pool_mb=pool_mb)
+    out = [frame(r, f) for i in range(70)]
+    r.set_precision(MIXED, pool_mb=pool_mb)
+    return out, frame(r, f)[2]
+limited, again = run(2.0)
+rt.fake_memory(rt.fake_held() + (300 << 20))
+free, _ = run(0.0)
+print(json.dumps([grown, free, limited, again]))
+""")
+    assert 1.8 * grown[0] < grown[1] < 2.2 * grown[0] and 1.8 * grown[1] < grown[2] < 2.2 * grown[1]
+    for frames in (free, limited):
+        assert all(rc == 0 for rc, _, _ in frames)
+        assert all(m == 0 and n == frames[0][2] - 6 for _, m, n in frames[2:])
+    assert again == limited[0][2]
