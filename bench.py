@@ -313,7 +313,7 @@ def run_ours(args, so, world, rank, local):
     # the deferred form an FP32 tracer launch beyond the first, the mode sums (torus) and the transfer
     waves = max(st.record_waves, 1)
     mixed_launches = 7 + (waves - 1) + (waves * ((1 if st.turb_records > 0 else 0) + 1) if st.record_waves > 0 else 0)
-    if flow:  # band and re-trace: recording pass, emission, transfer and replay launch each
+    if flow and st.rec64_slots:  # band and re-trace deferred: recording pass, emission, transfer, replay launch each
         mixed_launches += 6
     gpu_launches = args.steps * ((plain_launches if path == "fp64" else mixed_launches) + (1 if flow else 0))
     if flow:

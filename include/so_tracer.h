@@ -180,7 +180,9 @@ typedef struct so_stats {
     double ms_sum64;      /* ... of the FP64 turbulence sums over all records (k_turb64_records) */
     double ms_replay64;   /* ... of the replay pass (geodesic again, sums read back, emission); with
                              deferred emission it runs only when the record pool ran out */
-    long long rec64_slots; /* ... record slots summed (segments taken x 16) */
+    long long rec64_slots; /* ... record slots summed (segments taken x 16); on a mixed frame this and the
+                              * next two count the passes of its band and re-traced rays too (0 where
+                              * those ran in the tracer) */
     long long rec64_short; /* ... samples summed in the tracer because the record pool ran out */
     long long rec64_records; /* ... records written (flow steps that needed a sum, up to each ray's end) */
     double ms_emit64;     /* ... deferred emission: device time of the emission at every record and the

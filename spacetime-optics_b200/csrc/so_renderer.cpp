@@ -180,7 +180,7 @@ struct so_renderer {
     bool side_bounded = false;                 // the last such frame's pool was smaller than its need
     unsigned long long* h_side = nullptr;      // pinned: pool counters of the two launches (3 each)
     cudaEvent_t ev_side = nullptr;
-    bool side_pending = false;
+    bool side_pending = false, last_side = false;
     long long list_rays = 0;                   // rays of the last so_trace_rays whose counters d_cnt holds
     std::vector<so_batch*> batches;            // live batches on this renderer (detached by so_destroy)
     std::string err;
@@ -1033,6 +1033,7 @@ int trace_pass1_mixed(so_renderer* r, const so_frame& f, TraceLaunch& L) {
         side = rays < 0.25 * (double)ns + 4096.0 && ensure_side(r, (long long)std::min(rays, (double)ns), ns) == SO_OK;
         if (!side) r->err.clear();
     }
+    r->last_side = side;
     int rc = run_side(r, Lb, side, 0);
     if (rc) return rc;
     const bool torus_defer = variant_of(r->S) == VAR_RADIO && L.torus && L.n_modes > 0;
@@ -1292,6 +1293,13 @@ int trace_frame(so_renderer* r, const so_frame& f, bool adaptive, so_stats* stat
             c.fp64_rays = 0;
         }
         rec64_stats(r, stats);
+        if (mixed && r->last_side) {  // the band and the re-trace
+            for (int k = 0; k < 6; k += 3) {
+                stats->rec64_slots += (long long)std::min<unsigned long long>(r->h_side[k], r->side.seg_cap) * REC_SEG;
+                stats->rec64_short += (long long)r->h_side[k + 1];
+                stats->rec64_records += (long long)r->h_side[k + 2];
+            }
+        }
         float ms1 = 0.f, ms2 = 0.f;
         cudaEventElapsedTime(&ms1, ev[0], ev[1]);
         if (cudaEventQuery(ev[3]) == cudaSuccess && cudaEventElapsedTime(&ms2, ev[2], ev[3]) != cudaSuccess) ms2 = 0.f;
