@@ -1756,7 +1756,9 @@ int so_set_precision(so_renderer* r, int precision, const so_mixed_opts* opts) {
     r->precision = precision;
     if (opts) {
         r->mixed = *opts;
-        r->side_max_rays = 0x7fffffffffffffffll;  // another limit, band or depth
+        // another limit, band or depth: what the last frame's side passes found does not count
+        r->side_max_rays = 0x7fffffffffffffffll;
+        r->side_pending = false;
     }
     return SO_OK;
 }

@@ -147,3 +147,21 @@ print(json.dumps([grown, free, limited, again]))
         assert all(rc == 0 for rc, _, _ in frames)
         assert all(m == 0 and n == frames[0][2] - 6 for _, m, n in frames[2:])
     assert again == limited[0][2]
+
+
+def test_shortage_under_other_options_is_forgotten(host):
+    """A shortage under pool_mb = 2 says nothing about the pool that so_set_precision allows next: the first frame
+    after it defers, with the launches of a new renderer's first frame."""
+    new, after = host("""
+rt.fake_counts(1, 1, 1, 1)
+r, f = flow(64)
+r.set_precision(MIXED, pool_mb=64.0)
+new = frame(r, f)
+r.close()
+r, f = flow(64)
+r.set_precision(MIXED, pool_mb=2.0)
+frame(r, f)
+r.set_precision(MIXED, pool_mb=64.0)
+print(json.dumps([new, frame(r, f)]))
+""")
+    assert new[0] == after[0] == 0 and new[2] == after[2]
