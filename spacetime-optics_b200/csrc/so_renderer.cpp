@@ -183,6 +183,7 @@ struct so_renderer {
     bool side_pending = false, last_side = false;
     long long list_rays = 0;                   // rays of the last so_trace_rays whose counters d_cnt holds
     std::vector<so_batch*> batches;            // live batches on this renderer (detached by so_destroy)
+    unsigned buffers_gen = 0;                  // counts replacements of buffers that a batch's graph points at
     std::string err;
 };
 
@@ -523,13 +524,18 @@ int ensure_records64(so_renderer* r, long long jobs, int per_job, int w, long lo
     const double seg_doubles = (double)REC_SEG * w;
     const double per_seg = seg_doubles * sizeof(double) + sizeof(uint32_t) + sizeof(uint2);
     const double seg_per_job = (r->rec_per_sample64 / REC_SEG + 1.0) * per_job;  // a partly filled segment per sample
-    long long want = std::min<long long>((long long)std::ceil((double)jobs * seg_per_job), 0x7fffffffll);
+    long long limit = 0x7fffffffll;
     if (r->mixed.pool_mb > 0.0)
-        want = std::min<long long>(want, std::max<long long>(1, (long long)(r->mixed.pool_mb * 1048576.0 / per_seg)));
+        limit = std::min<long long>(limit, std::max<long long>(1, (long long)(r->mixed.pool_mb * 1048576.0 / per_seg)));
+    const long long want = std::min<long long>((long long)std::ceil((double)jobs * seg_per_job), limit);
     const long long want_d = (long long)(want * seg_doubles);
-    if (r->rec64_doubles <= 0 || want_d > r->pool64_target ||
-        (r->mixed.pool_mb > 0.0 && want_d < r->rec64_doubles)) {
+    // grow to a larger estimate; shrink only to a lowered limit (launches of different sizes and record widths
+    // share the pool)
+    const bool over = r->mixed.pool_mb > 0.0 &&
+                      (double)r->rec64_doubles > std::max(r->mixed.pool_mb * 1048576.0 / sizeof(double), seg_doubles);
+    if (r->rec64_doubles <= 0 || want_d > r->pool64_target || over) {
         SO_CK(r, cudaStreamSynchronize(r->st));
+        ++r->buffers_gen;
         if (r->d_rec64) cudaFree(r->d_rec64);
         if (r->d_seg_next64) cudaFree(r->d_seg_next64);
         if (r->d_seg_meta64) cudaFree(r->d_seg_meta64);
@@ -562,6 +568,7 @@ int ensure_records64(so_renderer* r, long long jobs, int per_job, int w, long lo
     *wave_jobs = wave;
     const long long heads = wave * per_job;  // one chain per sample
     if (heads > r->job_cap64) {
+        ++r->buffers_gen;
         if (r->d_job_head64) cudaFree(r->d_job_head64);
         if (r->d_samp64) cudaFree(r->d_samp64);
         r->d_job_head64 = nullptr;
@@ -1772,6 +1779,7 @@ int so_set_plasma(so_renderer* r, const so_plasma* p, const so_mode* modes) {
         if (!(p->h_sph > 0)) return fail(r, SO_ERR_ARG, "h_sph must be > 0");
     }
     if (cudaSetDevice(r->device) != cudaSuccess) return fail(r, SO_ERR_CUDA, "cudaSetDevice");
+    ++r->buffers_gen;
     if (r->d_modes) {
         cudaFree(r->d_modes);
         r->d_modes = nullptr;
@@ -1918,6 +1926,7 @@ struct so_batch {
     cudaGraphExec_t gexec = nullptr;
     float* graph_px = nullptr;  // output buffer baked into the graph
     so_tune graph_tune{-1, -1, 0.0, -1, -1};
+    unsigned graph_gen = 0;     // the renderer's buffers_gen it was captured with
     // deferred passes (radio frames without disks): decided and sized before each graph capture;
     // wave64 = 0 traces in one persistent launch
     bool defer_ok = false;
@@ -2048,6 +2057,7 @@ int batch_capture(so_batch* b, float* d_px) {
     SO_CK(r, cudaGraphInstantiate(&b->gexec, g, 0));
     b->graph_px = d_px;
     b->graph_tune = b->tune;
+    b->graph_gen = r->buffers_gen;
     return SO_OK;
 }
 
@@ -2137,7 +2147,9 @@ int so_batch_render(so_batch* b, float* d_px, so_stats* stats) {
         }
         cudaGetLastError();  // a pending event reports cudaErrorNotReady
     }
-    if (!b->gexec || b->graph_px != d_px || !same_tune(b->graph_tune, b->tune)) {
+    // (a graph keeps the pointers of its launches: the record pool may have been replaced by a larger frame's or
+    // batch's, the modes by so_set_plasma)
+    if (!b->gexec || b->graph_px != d_px || !same_tune(b->graph_tune, b->tune) || b->graph_gen != r->buffers_gen) {
         int rc = batch_capture(b, d_px);
         if (rc) return rc;
     }

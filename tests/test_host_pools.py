@@ -165,3 +165,40 @@ r.set_precision(MIXED, pool_mb=64.0)
 print(json.dumps([new, frame(r, f)]))
 """)
     assert new[0] == after[0] == 0 and new[2] == after[2]
+
+
+BATCH = """
+def batch(r, f, size, frames):
+    px = np.zeros(frames * size * size * 4, np.float32)
+    b = so.Batch(r, [r.scene], [f] * frames, [0] * frames, size, size)
+    def render():
+        g = rt.fake_graphs()
+        st = b.render(px.ctypes.data, stats=True)
+        return rt.fake_graphs() - g, st.rec64_waves
+    return render
+"""
+
+
+def test_batch_graph_follows_its_buffers(host):
+    """A batch's graph holds the pointers of its launches, so it is captured again when the record pool has been
+    replaced (a larger frame or batch on the renderer) or the modes (so_set_plasma), and only then: two
+    batches under one pool_mb do not replace each other's pool."""
+    got = host(BATCH + """
+r, f = flow(128)
+r.set_precision(FP64)
+a = batch(r, f, 32, 5)
+out = [a()[0], a()[0], frame(r, f)[0], a()[0], frame(r, f)[0], a()[0]]
+sh = so.Shot("synchrotron_1024.ini", ["so.modes=8", "camera.width=32", "camera.height=32"])
+t = so.Renderer(sh.scene, sh.tables, sh.settings)
+t.set_plasma(sh.plasma())
+b = batch(t, sh.frame(0), 32, 5)
+out += [b()[0], b()[0]]
+t.set_plasma(sh.plasma())
+out += [b()[0], b()[0]]
+r.set_precision(FP64, pool_mb=64.0)
+c, d = batch(r, f, 32, 5), batch(r, f, 32, 12)
+c(), d(), c(), d()
+out += [c()[0], d()[0], c()[0], d()[0]]
+print(json.dumps(out))
+""")
+    assert got == [1, 0, 0, 1, 0, 0, 1, 0, 1, 0, 0, 0, 0, 0]
