@@ -1930,7 +1930,7 @@ struct so_batch {
     // deferred passes (radio frames without disks): decided and sized before each graph capture;
     // wave64 = 0 traces in one persistent launch
     bool defer_ok = false;
-    long long wave64 = 0;
+    long long wave64 = 0, seg_cap64 = 0;  // jobs per wave, the pool's segments
     int sums64 = 0;              // 0 none (reference flow, torus without modes), 1 FP64, 2 FP32 (mixed)
     int w64 = REC64_W_TORUS;     // doubles per record
 };
@@ -2014,9 +2014,9 @@ void batch_plan(so_batch* b, float* d_px) {
         return;
     }
     b->wave64 = wave;
+    b->seg_cap64 = r->seg_cap64;
     b->w64 = w;
     b->sums64 = !sums ? 0 : (r->precision == SO_PREC_MIXED && r->turb_modes) ? 2 : 1;
-    r->samples64 = L.nrays * b->spp;
 }
 
 // The launch sequence of one batch: counter reset, the tracer over all frames (one persistent launch,
@@ -2030,7 +2030,6 @@ int batch_enqueue(so_batch* b, float* d_px) {
         if (int rc = enqueue_deferred64(r, main_records(r), L, b->variant, r->st, b->wave64, b->w64, b->sums64, true,
                                         false, r->h_rec64))
             return rc;
-        r->waves64 = (int)((L.nrays + b->wave64 - 1) / b->wave64);
     } else {
         cudaError_t e = launch_trace64(L, b->variant, r->num_sms, r->st);
         if (e != cudaSuccess) return cuda_fail(r, e, "batch tracer launch");
@@ -2165,7 +2164,10 @@ int so_batch_render(so_batch* b, float* d_px, so_stats* stats) {
         if (e1) cudaEventDestroy(e1);
         return cuda_fail(r, e, "so_batch_render graph launch");
     }
-    if (b->wave64 > 0) {  // the graph copied each wave's pool counters out: note when they are there
+    if (b->wave64 > 0) {  // the graph copies each wave's pool counters out: how many, and when they are there
+        const long long jobs = (long long)b->W * b->H * b->nframes;
+        r->waves64 = (int)((jobs + b->wave64 - 1) / b->wave64);
+        r->samples64 = jobs * b->spp;
         cudaEventRecord(r->ev_rec64, r->st);
         r->rec64_pending = true;
     }
@@ -2190,7 +2192,7 @@ int so_batch_render(so_batch* b, float* d_px, so_stats* stats) {
         if (b->wave64 > 0) {  // the deferred passes' pool counters, copied out by the graph
             unsigned long long slots = 0, short_samples = 0, records = 0;
             for (int k = 0; k < r->waves64; ++k) {
-                slots += std::min<unsigned long long>(r->h_rec64[3 * k], (unsigned long long)r->seg_cap64) * REC_SEG;
+                slots += std::min<unsigned long long>(r->h_rec64[3 * k], (unsigned long long)b->seg_cap64) * REC_SEG;
                 short_samples += r->h_rec64[3 * k + 1];
                 records += r->h_rec64[3 * k + 2];
             }

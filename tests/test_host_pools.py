@@ -202,3 +202,20 @@ out += [c()[0], d()[0], c()[0], d()[0]]
 print(json.dumps(out))
 """)
     assert got == [1, 0, 0, 1, 0, 0, 1, 0, 1, 0, 0, 0, 0, 0]
+
+
+def test_batch_counts_its_own_waves(host):
+    """A batch in waves reports (and looks for shortages in) its own number of waves, also when the renderer traced
+    a frame in another number since its graph was captured."""
+    got = host(BATCH + """
+r, f = flow(72)
+r.set_precision(FP64, pool_mb=100.0)
+b = batch(r, f, 32, 20)
+first = b()[1]
+st = so.abi.Stats()
+px = np.zeros(72 * 72 * 4, np.float32)
+so.lib().so_render_device(r.h, C.byref(f), px.ctypes.data_as(C.c_void_p), C.byref(st))
+print(json.dumps([first, st.rec64_waves, b()]))
+""")
+    first, between, (graphs, again) = got
+    assert first > 1 and between != first and graphs == 0 and again == first
