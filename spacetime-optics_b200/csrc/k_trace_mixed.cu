@@ -1089,12 +1089,18 @@ cudaError_t launch_sky_escape(const TraceLaunch& L, int num_sms, cudaStream_t st
     return cudaGetLastError();
 }
 
-void turb_modes_fold(const so_mode* modes, int n, TurbModes* out) {
+void turb_modes_fold(const so_mode* modes, int n, double r_max, TurbModes* out) {
+    bool near = true;  // (false for a NaN)
+    for (int i = 0; i < n; ++i) {
+        const so_mode& m = modes[i];
+        near = near && sqrt(m.kx * m.kx + m.ky * m.ky + m.kz * m.kz) * r_max < 1048576.0 * 2.0 * PI;
+    }
     out->n = n;
+    out->grouped = near ? n : 0;
     for (int i = 0; i < n; ++i) {
         const so_mode& m = modes[i];
         const double ph = m.phase - 2.0 * PI * floor(m.phase / (2.0 * PI) + 0.5);
-        const bool poly = i % TURB_POLY == TURB_POLY - 1;
+        const bool poly = near && i % TURB_POLY == TURB_POLY - 1;
         const double f = poly ? 0.5 / PI : 1.0;
         out->k[i] = make_float4((float)(m.kx * f), (float)(m.ky * f), (float)(m.kz * f), (float)(ph * f));
         out->a[i] = (float)m.amp;

@@ -243,15 +243,17 @@ cudaError_t launch_mip_half2(cudaSurfaceObject_t src, int sw, int sh, cudaSurfac
                              cudaStream_t st);
 // Fourier modes of the torus turbulence in FP32 (phase folded into (-pi, pi]), passed to the batched
 // sums as a kernel parameter (constant memory; up to SO_MAX_MODES = 1024, 20 KB).  The last of every
-// complete group of TURB_POLY modes has its wave vector and phase in turns (its cosine is taken on
-// the FMA pipe, so_packed32.cuh).
+// complete group of TURB_POLY among the first `grouped` modes has its wave vector and phase in turns (its
+// cosine is taken on the FMA pipe, so_packed32.cuh).  grouped = n, or 0 where a phase k . X + p, |X| <= r_max,
+// could leave that cosine's range (2^21 turns; half of it here): beyond, its polynomial is unbounded,
+// while the SFU's cosine of such a phase, all rounding as it is, still lies in [-1, 1].
 constexpr int TURB_POLY = 8;
 struct TurbModes {
     float4 k[SO_MAX_MODES];  // kx, ky, kz, phase
     float a[SO_MAX_MODES];   // amplitude
-    int n;
+    int n, grouped;
 };
-void turb_modes_fold(const so_mode* modes, int n, TurbModes* out);
+void turb_modes_fold(const so_mode* modes, int n, double r_max, TurbModes* out);
 cudaError_t launch_turb_records(const TraceLaunch& L, const TurbModes& M, int num_sms, cudaStream_t st);
 // FP32 sums (SFU) at every record of a defer64 = 1 pass: the mixed form of launch_turb64_records.
 cudaError_t launch_turb32_rec64(const TraceLaunch& L, const TurbModes& M, int num_sms, cudaStream_t st);

@@ -65,7 +65,7 @@ __device__ __forceinline__ F2 cos_turns2(F2 t) {
 // 133.7 -> 121.2 ms, SFU pipe 87 %, FMA pipe 73 % (4.6 T cosines/s).
 template <int NP>
 __device__ __forceinline__ void mode_sums2(const TurbModes& M, const F2* x, const F2* y, const F2* z, F2* acc) {
-    const int nm = M.n;
+    const int nm = M.n, grouped = M.grouped;
     auto phase = [&](const float4& k, int q) {
         return fma2(both(k.z), z[q], fma2(both(k.y), y[q], fma2(both(k.x), x[q], both(k.w))));
     };
@@ -81,7 +81,7 @@ __device__ __forceinline__ void mode_sums2(const TurbModes& M, const F2* x, cons
     };
     int m = 0;
 #pragma unroll 1
-    for (; m + TURB_POLY <= nm; m += TURB_POLY) {
+    for (; m + TURB_POLY <= grouped; m += TURB_POLY) {
 #pragma unroll
         for (int j = 0; j < TURB_POLY - 1; ++j) sfu(m + j);
         const float4 k = M.k[m + TURB_POLY - 1];

@@ -92,7 +92,9 @@ struct so_renderer {
     // plasma / precision
     so_plasma plasma{};
     so_mode* d_modes = nullptr;
-    TurbModes* turb_modes = nullptr;  // the modes folded to FP32 for the batched turbulence sums
+    std::vector<so_mode> modes;       // host copy of d_modes
+    TurbModes* turb_modes = nullptr;  // the modes folded to FP32 for the batched turbulence sums (fold_modes)
+    double turb_r_max = -1.0;         // the radius they were folded for
     int precision = SO_PREC_FP64;
     so_mixed_opts mixed{0.05, 3e-6, 0.0, 1e-4, 0.0, 0.0, 0, 0, 0, 0.0, 0, 0.0, 0};
     // deferred turbulence: record pool (segments of REC_SEG slots), grown when a frame runs out
@@ -447,6 +449,15 @@ void launch_common(so_renderer* r, TraceLaunch& L) {
     L.drift_tol = r->mixed.drift_tol;
 }
 
+// The modes folded for FP32 sums at radii up to r_max.
+const TurbModes& fold_modes(so_renderer* r, double r_max) {
+    if (r->turb_r_max != r_max) {
+        turb_modes_fold(r->modes.data(), (int)r->modes.size(), r_max, r->turb_modes);
+        r->turb_r_max = r_max;
+    }
+    return *r->turb_modes;
+}
+
 // Buffers of the device luminance statistics (allocated on the first so_render).
 int ensure_lum(so_renderer* r) {
     if (r->lum.lum) return SO_OK;
@@ -601,9 +612,10 @@ Records64 main_records(const so_renderer* r) {
 // ensure_records64 set up: per wave a recording pass, the sums (sums: 0 none, 1 FP64, 2 FP32), the
 // emission and ordered transfer (emit), and a replay pass that runs when the pool ran short (always,
 // without emit).  With `timed` the phases are bracketed by events (not inside a graph capture).
-// Each wave's pool counters go to `ctl` (3 per wave).
+// Each wave's pool counters go to `ctl` (3 per wave).  r_max: the largest radius of a record (FP32 sums).
 int enqueue_deferred64(so_renderer* r, const Records64& pool, const TraceLaunch& L, int var, cudaStream_t s,
-                       long long wave, int w, int sums, bool emit, bool timed, unsigned long long* ctl) {
+                       long long wave, int w, int sums, bool emit, bool timed, unsigned long long* ctl,
+                       double r_max) {
     const int nw = (int)((L.nrays + wave - 1) / wave);
     if (nw > kMaxWaves64) return fail(r, SO_ERR_SIZE, "FP64 record pool: too many waves");
     if (timed) {
@@ -642,7 +654,7 @@ int enqueue_deferred64(so_renderer* r, const Records64& pool, const TraceLaunch&
         if (e != cudaSuccess) return cuda_fail(r, e, "tracer launch (recording pass)");
         if (ev) cudaEventRecord(ev[1], s);
         if (sums == 1) e = launch_turb64_records(L1, r->num_sms, s);
-        else if (sums == 2) e = launch_turb32_rec64(L1, *r->turb_modes, r->num_sms, s);
+        else if (sums == 2) e = launch_turb32_rec64(L1, fold_modes(r, r_max), r->num_sms, s);
         if (e != cudaSuccess) return cuda_fail(r, e, "deferred turbulence sums");
         if (ev) cudaEventRecord(ev[2], s);
         if (emit) {
@@ -681,7 +693,7 @@ int run_tracer(so_renderer* r, const TraceLaunch& L, cudaStream_t st = nullptr) 
         if (ensure_records64(r, L.nrays, per_job, w, &wave) == SO_OK) {
             r->samples64 = L.nrays * per_job;
             if (int rc = enqueue_deferred64(r, main_records(r), L, var, s, wave, w, torus ? 1 : 0, emit_ok, true,
-                                            r->h_rec64))
+                                            r->h_rec64, r->S.r_flow_max))
                 return rc;
             r->waves64 = (int)((L.nrays + wave - 1) / wave);
             SO_CK(r, cudaEventRecord(r->ev_rec64, s));
@@ -773,7 +785,7 @@ int run_side(so_renderer* r, const TraceLaunch& L, bool deferred, int slot) {
     if (!deferred) return run_tracer(r, L, r->st2);
     r->last_defer64 = false;
     return enqueue_deferred64(r, r->side, L, VAR_RADIO, r->st2, L.nrays, REC64_W_FLOW, 0, true, false,
-                              r->h_side + 3 * slot);
+                              r->h_side + 3 * slot, r->S.r_flow_max);
 }
 
 // Escape (u, v) of the (W + 1) x (H + 1) pixel corners of the frame in d_frame (k_corners,
@@ -1096,7 +1108,7 @@ int trace_pass1_mixed(so_renderer* r, const so_frame& f, TraceLaunch& L) {
         }
         if (defer) {
             SO_CK(r, cudaEventRecord(r->ev_wave[3 * w + 1], r->st));
-            if (torus_defer) SO_CK(r, launch_turb_records(Lw, *r->turb_modes, r->num_sms, r->st));
+            if (torus_defer) SO_CK(r, launch_turb_records(Lw, fold_modes(r, r->S.r_flow_max), r->num_sms, r->st));
             SO_CK(r, cudaEventRecord(r->ev_wave[3 * w + 2], r->st));
             SO_CK(r, launch_flow_records(Lw, r->num_sms, r->st));
         }
@@ -1788,8 +1800,9 @@ int so_set_plasma(so_renderer* r, const so_plasma* p, const so_mode* modes) {
     if (p->model == SO_PLASMA_TORUS && p->n_modes > 0) {
         if (dalloc(&r->d_modes, (size_t)p->n_modes) != cudaSuccess) return fail(r, SO_ERR_ALLOC, "modes alloc");
         SO_CK(r, cudaMemcpy(r->d_modes, modes, (size_t)p->n_modes * sizeof(so_mode), cudaMemcpyHostToDevice));
+        r->modes.assign(modes, modes + p->n_modes);
+        r->turb_r_max = -1.0;
         if (!r->turb_modes) r->turb_modes = new TurbModes;
-        turb_modes_fold(modes, p->n_modes, r->turb_modes);
     }
     return SO_OK;
 }
@@ -1930,6 +1943,7 @@ struct so_batch {
     // deferred passes (radio frames without disks): decided and sized before each graph capture;
     // wave64 = 0 traces in one persistent launch
     bool defer_ok = false;
+    double r_flow_max = 0.0;     // the largest of its scenes'
     long long wave64 = 0, seg_cap64 = 0;  // jobs per wave, the pool's segments
     int sums64 = 0;              // 0 none (reference flow, torus without modes), 1 FP64, 2 FP32 (mixed)
     int w64 = REC64_W_TORUS;     // doubles per record
@@ -2028,7 +2042,7 @@ int batch_enqueue(so_batch* b, float* d_px) {
     batch_launch_desc(b, d_px, L);
     if (b->wave64 > 0) {
         if (int rc = enqueue_deferred64(r, main_records(r), L, b->variant, r->st, b->wave64, b->w64, b->sums64, true,
-                                        false, r->h_rec64))
+                                        false, r->h_rec64, b->r_flow_max))
             return rc;
     } else {
         cudaError_t e = launch_trace64(L, b->variant, r->num_sms, r->st);
@@ -2087,6 +2101,7 @@ int so_batch_create(so_renderer* r, const so_scene* scenes, int nscenes, const s
     for (int s = 0; s < nscenes; ++s)
         b->defer_ok = b->defer_ok && scenes[s].mode == SO_MODE_RADIO && scenes[s].flow_on && !scenes[s].disk_on &&
                       scenes[s].max_steps < (1 << REC64_COUNT_BITS);
+    for (int s = 0; s < nscenes; ++s) b->r_flow_max = std::max(b->r_flow_max, scenes[s].r_flow_max);
     b->nframes = nframes;
     b->nscenes = nscenes;
     b->W = W;
