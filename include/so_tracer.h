@@ -560,6 +560,10 @@ int so_probe_sfu_peak(int device, double* gops);
  * at n phases d_t[i] into d_out[i] (device arrays, current device; synchronous): for checking it
  * against the CPU oracle's restatement. */
 int so_probe_cos_turns(const double* d_t, double* d_out, long long n);
+/* The tracers' straight-line arithmetic on the device, for checking it against the IEEE operators: op 0
+ * 1 / a, 1 a / b, 2 sqrt(a) of the FP64 tracer, 3 the FP32 tracer's 1 / (float)a (n operands in device
+ * arrays, d_b read by op 1 only, current device; synchronous). */
+int so_probe_quick(int op, const double* d_a, const double* d_b, double* d_out, long long n);
 
 /* ---- analytic helpers (kerr.hpp) --------------------------------------------------------------- */
 /* kerr_point (kerr.hpp:27-42). */

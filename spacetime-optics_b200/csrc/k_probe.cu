@@ -6,6 +6,11 @@
 #include "../../include/so_tracer.h"
 #include "so_kerr.cuh"
 
+namespace so {
+cudaError_t launch_quick64(int op, const double* a, const double* b, double* out, long long n);
+cudaError_t launch_quick32(const double* a, double* out, long long n);
+}  // namespace so
+
 namespace {
 template <typename T>
 __global__ void __launch_bounds__(256) k_fma_chains(T* out, int iters, T a, T b) {
@@ -112,4 +117,11 @@ extern "C" int so_probe_cos_turns(const double* d_t, double* d_out, long long n)
     if (n == 0) return SO_OK;
     k_cos_turns<<<592, 256>>>(d_t, d_out, n);
     return cudaGetLastError() == cudaSuccess && cudaDeviceSynchronize() == cudaSuccess ? SO_OK : SO_ERR_CUDA;
+}
+
+extern "C" int so_probe_quick(int op, const double* d_a, const double* d_b, double* d_out, long long n) {
+    if (op < 0 || op > 3 || n < 0 || (n > 0 && (!d_a || !d_out || (op == 1 && !d_b)))) return SO_ERR_ARG;
+    if (n == 0) return SO_OK;
+    const cudaError_t e = op == 3 ? so::launch_quick32(d_a, d_out, n) : so::launch_quick64(op, d_a, d_b, d_out, n);
+    return e == cudaSuccess && cudaDeviceSynchronize() == cudaSuccess ? SO_OK : SO_ERR_CUDA;
 }

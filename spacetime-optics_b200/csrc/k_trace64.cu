@@ -1250,4 +1250,15 @@ cudaError_t launch_trace64(const TraceLaunch& L, int variant, int num_sms, cudaS
     }
 }
 
+// The arithmetic of so_fast64.cuh as this file compiles it (so_probe_quick).
+__global__ void k_quick64(int op, const double* __restrict__ a, const double* __restrict__ b, double* __restrict__ out,
+                          long long n) {
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+        out[i] = op == 0 ? fast_rcp(a[i]) : op == 1 ? fast_div(a[i], b[i]) : fast_sqrt(a[i]);
+}
+cudaError_t launch_quick64(int op, const double* a, const double* b, double* out, long long n) {
+    k_quick64<<<592, 256>>>(op, a, b, out, n);
+    return cudaGetLastError();
+}
+
 }  // namespace so

@@ -1177,4 +1177,14 @@ cudaError_t launch_trace32(const TraceLaunch& L, long long n, int variant, int n
     return e;
 }
 
+// rcp32 as this file compiles it (so_probe_quick).
+__global__ void k_quick32(const double* __restrict__ a, double* __restrict__ out, long long n) {
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+        out[i] = (double)rcp32((float)a[i]);
+}
+cudaError_t launch_quick32(const double* a, double* out, long long n) {
+    k_quick32<<<592, 256>>>(a, out, n);
+    return cudaGetLastError();
+}
+
 }  // namespace so
