@@ -202,7 +202,8 @@ __global__ void __launch_bounds__(NT) k_gemm_bf16(GemmArgs g, int BN, int BK, in
     fence_after();
 
     if (ok) {
-        // Epilogue in column blocks of cb = 32 (16 for a 16-wide tile), staged through shared memory
+        // Epilogue in column blocks of cb = 32 (16 for a 16-wide tile; cw = 16 for the last one of a tile
+        // that is an odd multiple of 16 wide), staged through shared memory
         // (the K-slice buffers are free now): each thread takes its row's accumulators from TMEM
         // (its TMEM lane), the values go to small shared tiles, and the block then stores whole
         // 16-byte row segments -- or, for the transposed outputs, whole column segments -- so every
@@ -226,14 +227,14 @@ __global__ void __launch_bounds__(NT) k_gemm_bf16(GemmArgs g, int BN, int BK, in
             const uint4* src = reinterpret_cast<const uint4*>(g.d_in + (long)(m0 + r) * g.ldd + n0 + c);
 #pragma unroll
             for (int i = 0; i < 4; ++i)
-                if (8 * i < cb) dv[i] = __ldg(src + i);
+                if (8 * i < cb && c + 8 * i < BN) dv[i] = __ldg(src + i);
         };
         if (EPI == EPI_GELU_BWD && group * cb < BN) load_d(group * cb);
         for (int c = group * cb; c < BN; c += cb * NG) {
-            const int n = n0 + c;
+            const int n = n0 + c, cw = BN - c < cb ? BN - c : cb;
 #pragma unroll
             for (int h = 0; h < 32; h += 16) {
-                if (h >= cb) break;
+                if (h >= cw) break;
                 float f[16];
                 tmem_ld16(lane_addr + c + h, f);
                 if (EPI == EPI_F32 || EPI == EPI_SPLIT) {
@@ -278,7 +279,7 @@ __global__ void __launch_bounds__(NT) k_gemm_bf16(GemmArgs g, int BN, int BK, in
             group_sync();
             if (EPI == EPI_F32 || EPI == EPI_SPLIT) {
                 float* base = g.out_f + (EPI == EPI_SPLIT ? blockIdx.z * g.split_stride : 0);
-                const int segs = cb / 4;
+                const int segs = cw / 4;
                 for (int w = gtid; w < BM * segs; w += 128) {
                     const int rr = w / segs, sg = w % segs;
                     *reinterpret_cast<float4*>(base + (long)(m0 + rr) * g.ldf + n + 4 * sg) =
@@ -286,7 +287,7 @@ __global__ void __launch_bounds__(NT) k_gemm_bf16(GemmArgs g, int BN, int BK, in
                 }
             }
             if (EPI == EPI_GELU || EPI == EPI_GELU_BWD) {
-                const int segs = cb / 8;
+                const int segs = cw / 8;
                 for (int w = gtid; w < BM * segs; w += 128) {
                     const int rr = w / segs, sg = w % segs;
                     if (g.out_b)
@@ -297,7 +298,7 @@ __global__ void __launch_bounds__(NT) k_gemm_bf16(GemmArgs g, int BN, int BK, in
                             *reinterpret_cast<const uint4*>(TG + rr * 40 + 8 * sg);
                 }
                 if (g.out_t) {
-                    for (int w = gtid; w < cb * (BM / 8); w += 128) {
+                    for (int w = gtid; w < cw * (BM / 8); w += 128) {
                         const int j = w / (BM / 8), sg = w % (BM / 8);
                         *reinterpret_cast<uint4*>(g.out_t + (long)(n + j) * g.ldot + m0 + 8 * sg) =
                             *reinterpret_cast<const uint4*>(TT + j * 136 + 8 * sg);

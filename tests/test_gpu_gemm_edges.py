@@ -29,3 +29,16 @@ def test_split_reduction_lengths(so, kps, N):
         for z in range(splits):
             part = slice(z * kps, (z + 1) * kps)
             assert _close(c[z], a[:, part], b[:, part]) and _close(t[z].T, a[:, part], b[:, part])
+
+
+@pytest.mark.parametrize("N", [48, 80, 112, 208])
+def test_odd_multiples_of_16_columns(so, N):
+    """A tile whose last column block is 16 wide: the product, and nothing written past it."""
+    import torch
+    a, b = _operands(256, N, 320, N)
+    for layout in range(3):
+        c = torch.full((256 * N + 256,), 7.0, device="cuda")
+        torch.cuda.synchronize()
+        assert so.lib().so_sur_gemm(a.data_ptr(), b.data_ptr(), None, c.data_ptr(), 256, N, 320, 1, layout) == 0
+        p = c[:256 * N].view(N, 256).T if layout == 2 else c[:256 * N].view(256, N)
+        assert _close(p, a, b) and bool((c[256 * N:] == 7.0).all())
