@@ -160,7 +160,8 @@ __device__ __forceinline__ int ray_attempt(Ray64& R, const Scene& H, const so_sc
     ++R.it;
     double hc = R.h;
     if (VAR == VAR_RADIO && H.flow_on && R.y[0] < H.r_flow_max) {
-        // the smaller of r / |r'| and max(sin, 0.05) / |u'|, compared by products (dp54_fast)
+        // the smaller of r / |r'| and max(sin, 0.05) / |u'|, compared by products (either, where they are
+        // within 2^-52 of each other)
         const double q0 = fabs(R.y[1]) + 1e-30, q1 = fabs(R.y[3]) + 1e-30, s5 = R.sn > 0.05 ? R.sn : 0.05;
         const bool rad = R.y[0] * q1 < s5 * q0;
         const double cap = H.step_frac * fast_div(rad ? R.y[0] : s5, rad ? q0 : q1);

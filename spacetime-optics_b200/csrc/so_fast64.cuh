@@ -1,19 +1,28 @@
 // so_fast64.cuh -- branch-free FP64 division, square root and swept angle for the geodesic integrator,
 // and the Dormand-Prince attempt built on them.
 //
-// What bounds the FP64 tracer is the dependent chain of one attempt, about 1500 instructions of which
-// a quarter went to the FP64 pipe: every `/` and sqrt() is a range test, a branch and a call behind it,
-// so the scheduler cannot overlap the two quotients of a right-hand side, nor the five of the error
-// norm, and the code of all of them does not fit the instruction cache.  Here they are straight-line:
+// What bounds the FP64 tracer is the dependent chain of one attempt, and with many rays the issue of its
+// instructions: 920 per attempt of a vacuum ray with the IEEE operators, 45 % of them on the FP64 pipe (ncu,
+// 65,536 rays).  Every `/` and sqrt() is a range test, a branch and a call behind it, so the scheduler
+// cannot overlap the two quotients of a right-hand side, nor the five of the error norm, and the code of
+// all of them does not fit the instruction cache.  Here they are straight-line (640, 58 %):
 //   1/d, a/b   a 20-bit hardware seed, one third-order (Halley) step to within an ulp, then
 //              Markstein's correction q + y (a - b q) with the residual exact in one fma (P. Markstein,
 //              "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J.
-//              R&D 34, 1990), which rounds correctly
-//              (a reciprocal of the one significand that is all ones excepted: an ulp there);
+//              R&D 34, 1990);
 //   sqrt       the same with the residual x - g^2.
-// The results are those of the IEEE operators as long as nothing leaves the normal range, so the
-// integrator takes the same steps bit for bit; dp54_fast looks at its result once, and an attempt
-// with an out-of-range operand anywhere (a pole, a diverging trial step) is taken again by dp54.
+// How they round, with operands and results in the normal range:
+//   1/d        to nearest, but for the one significand that is all ones (an ulp there);
+//   sqrt       to nearest, also for the operands whose roots lie nearest to a midpoint of two doubles;
+//   a/b        within an ulp.  Markstein's theorem wants y rounded to nearest, and y is good to an ulp: of
+//              quotients made to lie next to a midpoint (within 2^-50 ulp of it) one in two hundred goes
+//              the wrong way, of random ones none in some millions.  Rounding y first mends that for two
+//              more fma a quotient, which cost the thin-disk frame 2.9 %, the FP64 flow frame 1.2 %.
+// (tests/fast64_midpoints.cpp, tests/fast64_check.cpp; the device's own: tests/test_gpu_quick_arithmetic.py.)
+// The integrator takes the steps of the IEEE form, bit for bit in every test, unless such a quotient or a
+// near tie of the error norm (dp54_fast) comes up; that moves one error or derivative by an ulp.  dp54_fast
+// looks at its result once, and an attempt with an out-of-range operand anywhere (a pole, a diverging trial
+// step) is taken again by dp54.
 //
 // Measured on the B200, IEEE operators against this form, results identical: 65,536 vacuum rays
 // 4.11 -> 3.28 ms, 1,021 of them (the longest ray's chain) 2.08 -> 1.54 ms, 262,144 rays through the
@@ -46,7 +55,7 @@ SO_HD double near_rcp(double d, double y0) {
     const double e = fma(-d, y0, 1.0);
     return fma(y0, fma(e, e, e), y0);
 }
-// 1/d and a/b correctly rounded (y: near_rcp of the divisor).
+// 1/d rounded to nearest, a/b within an ulp and nearly always to nearest (y: near_rcp of the divisor; see above).
 SO_HD double round_rcp(double d, double y) { return fma(y, fma(-d, y, 1.0), y); }
 SO_HD double round_quot(double a, double b, double y) {
     const double q = a * y;
@@ -110,11 +119,12 @@ static __constant__ Tableau dp_tableau = SO_TABLEAU_VALUES;
 #define SO_TABLEAU(T) static const Tableau T = SO_TABLEAU_VALUES
 #endif
 
-// dp54() in the same arithmetic; *ok says whether every operand stayed in range (else the result is
+// dp54() in this arithmetic; *ok says whether every operand stayed in range (else the result is
 // not to be used).  The error norm is the largest of five quotients |e_i| / sc_i.  Rounding is
 // monotone, so it is the rounded quotient of the largest ratio, found by comparing products; the two
-// constant denominators tol and 4 tol share one candidate (the factor 4 is exact).  A NaN candidate
-// is passed over, as fmax does.  Four divisions fewer.
+// constant denominators tol and 4 tol share one candidate (the factor 4 is exact).  The products are
+// rounded too: of two ratios within 2^-52 of each other the smaller may be taken, and the error be an ulp
+// below dp54's.  A NaN candidate is passed over, as fmax does.  Four divisions fewer.
 template <bool TIME = true>
 SO_HD double dp54_fast(const RayC& c, const double* y, const double* k1, double h, double tol, double* yo,
                        double* k7, bool* ok) {
@@ -180,7 +190,7 @@ SO_HD double dp54_fast(const RayC& c, const double* y, const double* k1, double 
 static __device__ __noinline__ double dp54_again(const RayC* c, const double* yk, double h, double tol, double* yo) {
     return dp54(*c, yk, yk + 6, h, tol, yo, yo + 6);
 }
-// dp54() through the fast form: the same steps and the same error.
+// dp54() through the fast form.
 template <bool TIME>
 __device__ __forceinline__ double dp54_attempt(const RayC& c, const double* y, const double* k1, double h, double tol,
                                                double* yo, double* k7) {

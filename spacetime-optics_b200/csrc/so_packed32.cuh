@@ -35,8 +35,8 @@ __device__ __forceinline__ F2 mul2(F2 a, F2 b) {
 
 // cos(2 pi t) of two phases in turns, |t| < 2^21, on the FMA pipe: cos_turns (so_kerr.cuh) in FP32.  The nearest
 // half turn q/2 is read off 2t + 1.5 * 2^23 (parity in the low mantissa bit), g = t - q/2 is exact, and
-// cos(2 pi g), |g| <= 1/4, is a polynomial of degree 4 in g^2 (Chebyshev fit, 4.7e-8 with FP32
-// coefficients).
+// cos(2 pi g), |g| <= 1/4, is a polynomial of degree 4 in g^2 (Chebyshev fit, fit_cos_turns.py: 4.7e-8, with
+// coefficients rounded to FP32 1.1e-7, evaluated in FP32 1.9e-7).
 __device__ __forceinline__ F2 cos_turns2(F2 t) {
     const F2 s = fma2(t, both(2.f), both(12582912.f));
     const F2 q = add2(s, both(-12582912.f));
