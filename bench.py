@@ -46,6 +46,11 @@ SFU_ATTEMPT = 21
 SFU_FLOW = 20
 
 
+def batched_sfu_cosines(n_modes):
+    """SFU cosines per record of the batched FP32 sums: every eighth mode takes the FMA pipe (so_packed32.cuh)."""
+    return n_modes - n_modes // 8
+
+
 def load_package():
     if "spacetime_optics_b200" in sys.modules:
         return sys.modules["spacetime_optics_b200"]
@@ -260,18 +265,19 @@ def run_ours(args, so, world, rank, local):
                 "peak": round(fp64_peak, 3), "unit": "TFLOP/s", "kernel": "k_trace64", "kernel_ms": st.ms_kernel,
                 "per_launch": flops, "peak_source": "so_probe_fma_peak (measured FP64 FMA chains on this GPU)"}
     elif st.turb_records > 0:
-        # deferred turbulence: the batched mode sums dominate, one SFU cosine per Fourier mode per
-        # record slot (the FP32 tracer and the ordered transfer are listed beside it)
+        # deferred turbulence: the batched mode sums dominate, one cosine per Fourier mode per record
+        # slot, seven of eight on the SFU (the FP32 tracer and the ordered transfer are listed beside it)
         sfu_peak = so.probe_sfu_peak(local)
-        ops = st.turb_records * n_modes
+        ops = st.turb_records * batched_sfu_cosines(n_modes)
         roof = {"bound": "sfu", "achieved": round(ops / (st.ms_turb * 1e-3) / 1e9, 3), "peak": round(sfu_peak, 3),
                 "unit": "Gop/s", "kernel": "k_turb_records", "kernel_ms": st.ms_turb, "per_launch": ops,
                 "peak_source": "so_probe_sfu_peak (measured SFU cosine chains on this GPU)",
                 "fp32_tflops_peak": round(fp32_peak, 3), "tracer_k_trace32_ms": round(st.ms_fp32_trace, 3),
                 "transfer_k_flow_records_ms": round(st.ms_fp32 - st.ms_fp32_trace - st.ms_turb, 3),
-                "record_slots": st.turb_records}
+                "record_slots": st.turb_records,
+                "cosines_gops": round(st.turb_records * n_modes / (st.ms_turb * 1e-3) / 1e9, 3)}
         # DRAM bytes per record slot of k_turb_records from its ncu capture on the 512^2 frame
-        # (profiles/k_turb_records_synchrotron512.md: 1.347 GB for 68.16 M slots), scaled by this
+        # (profiles/kernels_b200_summary.md: 1.35 GB for 68.16 M slots), scaled by this
         # frame's slots; the algorithmic figure is 20 bytes per slot
         roof["traffic"] = round(19.77 * st.turb_records)
         roof["traffic_source"] = "ncu dram bytes per slot at 512^2 x this frame's record slots"
@@ -858,9 +864,10 @@ def run_wavefront(args, so, world, rank, local):
                            if st.rec64_waves else "k_trace64"),
                 "peak_source": "so_probe_fma_peak (measured FP64 FMA chains on this GPU)"}
     else:
-        # FP64 geometry, FP32 turbulence sums: the SFU cosines (one per mode per flow step) dominate
+        # FP64 geometry, FP32 turbulence sums: the cosines (one per mode per flow step) dominate; of the
+        # deferred sums' seven of eight are the SFU's
         sfu_peak = so.probe_sfu_peak(local)
-        ops = st.flow_steps * n_modes
+        ops = st.flow_steps * (batched_sfu_cosines(n_modes) if st.rec64_waves else n_modes)
         achieved = ops / (ms_step * 1e-3) / 1e9
         roof = {"bound": "sfu", "achieved": round(achieved, 3), "peak": round(sfu_peak, 3), "unit": "Gop/s",
                 "frac": round(achieved / sfu_peak, 4), "traffic": None,
