@@ -511,6 +511,9 @@ int ensure_side_queue(so_renderer* r) {
 // pass (the same result, slower).  A shortage doubles the estimate for the next traces.
 constexpr int kMaxWaves64 = 64;
 constexpr long long kDeferMinJobs = 4096;
+// Records that a ray of a deferred trace can have: its steps (max_steps is below).  The estimates stop there; a
+// pool that no doubling can make large enough would send them out of range.
+constexpr double kMaxRecords = 1 << REC64_COUNT_BITS;
 int ensure_records64(so_renderer* r, long long jobs, int per_job, int w, long long* wave_jobs) {
     if (!r->h_rec64) {
         SO_CK(r, cudaMallocHost((void**)&r->h_rec64, 3 * kMaxWaves64 * sizeof(unsigned long long)));
@@ -530,6 +533,7 @@ int ensure_records64(so_renderer* r, long long jobs, int per_job, int w, long lo
         }
         const double seen = r->samples64 > 0 ? 1.5 * (double)records / (double)r->samples64 : 0.0;
         r->rec_per_sample64 = std::max(short_samples > 0 ? 2.0 * r->rec_per_sample64 : r->rec_per_sample64, seen);
+        r->rec_per_sample64 = std::min(r->rec_per_sample64, kMaxRecords);
     }
     cudaGetLastError();  // a pending event reports cudaErrorNotReady
     const double seg_doubles = (double)REC_SEG * w;
@@ -870,7 +874,7 @@ int ensure_records(so_renderer* r, long long ns) {
     if (!r->ev_seg) SO_CK(r, cudaEventCreateWithFlags(&r->ev_seg, cudaEventDisableTiming));
     if (r->seg_pending && cudaEventQuery(r->ev_seg) == cudaSuccess) {
         r->seg_pending = false;
-        if (r->h_seg[1] > 0) r->rec_per_ray *= 2.0;
+        if (r->h_seg[1] > 0) r->rec_per_ray = std::max(r->rec_per_ray, std::min(2.0 * r->rec_per_ray, kMaxRecords));
     }
     cudaGetLastError();  // a pending event reports cudaErrorNotReady
     const double per_seg = REC_SEG * (sizeof(float4) + sizeof(float)) + sizeof(uint32_t);

@@ -15,7 +15,7 @@ std::map<void*, size_t> blocks;
 size_t total = size_t(64) << 30, held = 0;
 long long fail_in = -1;  // allocations until the one that fails
 unsigned long long pool_counts[3];  // what a pool's three counters read back as
-int counts_given = 0;
+size_t counts_given = 0;            // (device to host copies of this size)
 int last_error = Ok;
 long long n_malloc = 0, n_graphs = 0, n_launch = 0;
 uintptr_t serial = 0x1000;
@@ -50,7 +50,7 @@ int handle(void** p) {
     return Ok;
 }
 int copy(void* d, const void* s, size_t n, int kind) {
-    if (kind == 2 && n == sizeof pool_counts && counts_given) std::memcpy(d, pool_counts, n);
+    if (kind == 2 && n == counts_given) std::memcpy(d, pool_counts, n);
     else std::memcpy(d, s, n);
     return Ok;
 }
@@ -60,8 +60,8 @@ extern "C" {
 void fake_memory(size_t bytes) { total = bytes; }
 size_t fake_held() { return held; }
 void fake_fail_in(long long n) { fail_in = n; }
-void fake_counts(int on, unsigned long long segments, unsigned long long short_samples, unsigned long long records) {
-    counts_given = on;
+void fake_counts(size_t bytes, unsigned long long segments, unsigned long long short_samples, unsigned long long records) {
+    counts_given = bytes;  // 24: the pools of the FP64 passes, 16: that of the FP32 rays
     pool_counts[0] = segments;
     pool_counts[1] = short_samples;
     pool_counts[2] = records;

@@ -24,7 +24,7 @@ for name in ("fake_held", "fake_largest"):
     getattr(rt, name).restype = C.c_size_t
 rt.fake_memory.argtypes = [C.c_size_t]
 rt.fake_fail_in.argtypes = [C.c_longlong]
-rt.fake_counts.argtypes = [C.c_int] + [C.c_ulonglong] * 3
+rt.fake_counts.argtypes = [C.c_size_t] + [C.c_ulonglong] * 3
 MIXED, FP64 = so.abi.SO_PREC_MIXED, so.abi.SO_PREC_FP64
 def flow(n):
     sh = so.Shot("m87_reference_flow.ini", ["camera.width=%%d" %% n, "camera.height=%%d" %% n, "render.spp=1",
@@ -123,7 +123,7 @@ def test_side_pool_that_cannot_grow(host):
     pool_mb neither grows nor records in vain: from the second frame on the rays run in the tracer (six
     launches fewer a frame, three a list), until so_set_precision gives another limit."""
     grown, free, limited, again = host("""
-rt.fake_counts(1, 1, 1, 1)
+rt.fake_counts(24, 1, 1, 1)
 r, f = flow(64)
 r.set_precision(MIXED)
 grown = []
@@ -153,7 +153,7 @@ def test_shortage_under_other_options_is_forgotten(host):
     """A shortage under pool_mb = 2 says nothing about the pool that so_set_precision allows next: the first frame
     after it defers, with the launches of a new renderer's first frame."""
     new, after = host("""
-rt.fake_counts(1, 1, 1, 1)
+rt.fake_counts(24, 1, 1, 1)
 r, f = flow(64)
 r.set_precision(MIXED, pool_mb=64.0)
 new = frame(r, f)
@@ -219,3 +219,20 @@ print(json.dumps([first, st.rec64_waves, b()]))
 """)
     first, between, (graphs, again) = got
     assert first > 1 and between != first and graphs == 0 and again == first
+
+
+@pytest.mark.parametrize("prec,size", [("FP64", 24), ("MIXED", 16)])
+def test_estimates_stay_finite(host, prec, size):
+    """70 frames under a pool_mb too small for any of them double the estimate of records per ray or sample; it stays
+    within what a ray can have, so that the first frame without the limit gets a pool (it had overflowed)."""
+    largest, frames = host("""
+r, f = flow(72)
+r.set_precision(%s, pool_mb=0.001)
+rt.fake_counts(%d, 1, 1, 1)
+frames = [frame(r, f)[0] for i in range(70)]
+rt.fake_counts(0, 0, 0, 0)
+r.set_precision(%s)
+frames.append(frame(r, f)[0])
+print(json.dumps([rt.fake_largest(), frames]))
+""" % (prec, size, prec))
+    assert not any(frames) and largest > 1 << 28
