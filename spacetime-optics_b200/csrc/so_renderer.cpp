@@ -1795,15 +1795,21 @@ int so_set_plasma(so_renderer* r, const so_plasma* p, const so_mode* modes) {
         if (!(p->h_sph > 0)) return fail(r, SO_ERR_ARG, "h_sph must be > 0");
     }
     if (cudaSetDevice(r->device) != cudaSuccess) return fail(r, SO_ERR_CUDA, "cudaSetDevice");
-    ++r->buffers_gen;
-    if (r->d_modes) {
-        cudaFree(r->d_modes);
-        r->d_modes = nullptr;
+    so_mode* fresh = nullptr;
+    const bool summed = p->model == SO_PLASMA_TORUS && p->n_modes > 0;
+    if (summed) {
+        if (dalloc(&fresh, (size_t)p->n_modes) != cudaSuccess) return fail(r, SO_ERR_ALLOC, "modes alloc");
+        const cudaError_t e = cudaMemcpy(fresh, modes, (size_t)p->n_modes * sizeof(so_mode), cudaMemcpyHostToDevice);
+        if (e != cudaSuccess) {
+            cudaFree(fresh);
+            return cuda_fail(r, e, "modes upload");
+        }
     }
+    ++r->buffers_gen;
+    if (r->d_modes) cudaFree(r->d_modes);
+    r->d_modes = fresh;
     r->plasma = *p;
-    if (p->model == SO_PLASMA_TORUS && p->n_modes > 0) {
-        if (dalloc(&r->d_modes, (size_t)p->n_modes) != cudaSuccess) return fail(r, SO_ERR_ALLOC, "modes alloc");
-        SO_CK(r, cudaMemcpy(r->d_modes, modes, (size_t)p->n_modes * sizeof(so_mode), cudaMemcpyHostToDevice));
+    if (summed) {
         r->modes.assign(modes, modes + p->n_modes);
         r->turb_r_max = -1.0;
         if (!r->turb_modes) r->turb_modes = new TurbModes;

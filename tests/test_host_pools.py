@@ -236,3 +236,21 @@ frames.append(frame(r, f)[0])
 print(json.dumps([rt.fake_largest(), frames]))
 """ % (prec, size, prec))
     assert not any(frames) and largest > 1 << 28
+
+
+def test_refused_plasma_changes_nothing(host):
+    """so_set_plasma that cannot allocate its modes keeps the renderer's plasma, modes and all."""
+    rc, alloc, before, after, frames = host("""
+sh = so.Shot("synchrotron_1024.ini", ["so.modes=8", "camera.width=32", "camera.height=32"])
+r = so.Renderer(sh.scene, sh.tables, sh.settings)
+r.set_plasma(sh.plasma())
+first = frame(r, sh.frame(0))[0]
+held = rt.fake_held()
+p = sh.plasma()
+p.n_modes = 512
+rt.fake_fail_in(0)
+rc = so.lib().so_set_plasma(r.h, C.byref(p), so.plasma_modes(p))
+rt.fake_fail_in(-1)
+print(json.dumps([rc, so.abi.SO_ERR_ALLOC, held, rt.fake_held(), [first, frame(r, sh.frame(0))[0]]]))
+""")
+    assert rc == alloc and before == after and frames == [0, 0]
