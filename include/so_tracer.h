@@ -388,7 +388,8 @@ void so_destroy(so_renderer* r);
  * SO_PREC_MIXED, FP64 otherwise; none for the reference flow model, whose noise a batch evaluates
  * in place), the emission and the ordered transfer, in waves through the renderer's record pool
  * (sized before the capture, within so_mixed_opts.pool_mb); a batch that ran short of records is
- * captured again with a larger pool at its next so_batch_render. */
+ * captured again with a larger pool at its next so_batch_render, and so is one whose pool another
+ * launch on the renderer, or whose modes so_set_plasma, has replaced since. */
 typedef struct so_batch so_batch;
 /* Launch shape of the batch: resident CTAs per SM of the persistent grid (0 = as many as fit); the
  * job order (0 = frame after frame, 1 = frames interleaved in tiles of `tile` consecutive pixels,
